@@ -17,6 +17,7 @@
 #define NBCS_DETMATH_H
 
 #include <math.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define NBCS_HD __host__ __device__ __forceinline__
@@ -61,19 +62,35 @@ NBCS_HD double nbcs_sin_poly(double x)
     return x + x * (z * p);
 }
 
+/* the bit pattern, which orders nonnegative doubles (NaN above all): the range
+ * tests below then need no FP64 compare, 19 cycles of the GPU's FP64 pipe each */
+NBCS_HD unsigned long long nbcs_bits(double d)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned long long)__double_as_longlong(d);
+#else
+    unsigned long long u;
+    memcpy(&u, &d, sizeof u);
+    return u;
+#endif
+}
+
 NBCS_HD double nbcs_cos_deg(double d)
 {
     const double rad = 3.141592653589793 / 180.0;
-    double a = fabs(d);
-    if (!(a <= 1.0e15)) return a == a ? 1.0 : a; /* huge: give up gracefully; NaN -> NaN */
-    a = fmod(a, 360.0);                 /* exact */
-    if (a > 180.0) a = 360.0 - a;       /* exact (Sterbenz) */
-    double sgn = 1.0;
-    if (a > 90.0) {
-        a = 180.0 - a;                  /* exact */
-        sgn = -1.0;
+    double a = fabs(d), sgn = 1.0, r;
+    if (nbcs_bits(a) > 0x4056800000000000ull) {  /* above 90 degrees, or NaN */
+        if (!(a <= 1.0e15)) return a == a ? 1.0 : a; /* huge: give up gracefully; NaN -> NaN */
+        if (a >= 360.0) a = fmod(a, 360.0); /* exact; below 360 the remainder is a itself */
+        if (a > 180.0) a = 360.0 - a;       /* exact (Sterbenz) */
+        if (a > 90.0) {
+            a = 180.0 - a;                  /* exact */
+            sgn = -1.0;
+        }
     }
-    double r = (a <= 45.0) ? nbcs_cos_poly(a * rad) : nbcs_sin_poly((90.0 - a) * rad);
+    /* up to 45 degrees the cosine series, above it the sine of the complement */
+    if (nbcs_bits(a) <= 0x4046800000000000ull) r = nbcs_cos_poly(a * rad);
+    else r = nbcs_sin_poly((90.0 - a) * rad);
     return sgn * r;
 }
 

@@ -11,11 +11,15 @@
 
 namespace nbcs {
 
-// One 256-thread block per 32 x 8 tile of particles (warps of 4 x 8): as in
-// the mixed kernel, the warps of a block follow neighbouring trajectories and
-// share L1 lines (geophysical workload: 194 ms against 209 ms with one block
-// per 128 consecutive particles of a row).
-constexpr int kFm64Block = 256;
+// One warp per block, a 4 x 8 tile of particles.  The kernel is bound by the
+// FP64 pipe, which two or three warps a partition keep busy, so what counts is
+// an even share of the work: single-warp blocks are the finest unit that the
+// SMs can take from the launch.  Against 256-thread blocks (32 x 8 tiles), with
+// the operations that left the FP64 pipe in the same change: double gyre 401 x
+// 201 8.09 -> 5.45 ms, geophysical flow 338 x 126 (rtol 1e-6) 56.7 -> 31.3 ms
+// (176 blocks had kept the SMs busy 56 % of the time), 21 x 11 double gyre
+// 1.74 -> 1.02 ms.
+constexpr int kFm64Block = 32;
 
 template <class Flow>
 __global__ void __launch_bounds__(kFm64Block)
@@ -91,7 +95,7 @@ struct Launch64 {
 // per point of a list, the positions at the n output times teval by dense
 // output of one DOP853 run (16 stage slots per thread); masked points and the
 // outputs past a failure stay 0.
-constexpr int kDense64Block = 128;
+constexpr int kDense64Block = 32;
 
 template <class Flow>
 __global__ void __launch_bounds__(kDense64Block)

@@ -57,25 +57,35 @@ struct FlowBickley64 {
     }
 };
 
-// Python's float modulo (sign of the divisor), as numba evaluates `%`.
-__device__ __forceinline__ double py_fmod(double a, double b)
+// Python's float modulo a % 360 (sign of the divisor), as numba evaluates it.
+// For |a| < 360 -- every longitude that does not lap the globe within a stage
+// -- fmod returns its argument; the range test is on the bit pattern.
+__device__ __forceinline__ double py_mod360(double a)
 {
-    double m = fmod(a, b);
-    if (m != 0.0) {
-        if ((b < 0.0) != (m < 0.0)) m += b;
-    } else {
-        m = copysign(0.0, b);
-    }
-    return m;
+    const unsigned hi = (unsigned)(__double_as_longlong(a) >> 32);
+    double m = a;
+    if ((hi & 0x7fffffffu) >= 0x40768000u) m = fmod(a, 360.0);  // |a| >= 360, inf, NaN
+    const long long mb = __double_as_longlong(m);
+    if ((mb & 0x7fffffffffffffffll) == 0) return 0.0;
+    return mb < 0 ? m + 360.0 : m;  // NaN stays NaN
 }
 
+// Weights of the four cubic B-spline pieces at offset t:
+//   w0 = (-1/6) t^3 + (3/6) t^2 + (-3/6) t + (1/6)
+//   w1 =  (3/6) t^3 + (-6/6) t^2 + (0/6) t + (4/6)
+//   w2 = (-3/6) t^3 + (3/6) t^2 + (3/6) t + (1/6)
+//   w3 =  (1/6) t^3 + 0 + 0 + 0
+// in the reference's operation order.  Products with 1/2 and 1 are exact, so
+// they ride in the FMA of the sum that follows (one rounding, the sum's), the
+// zero terms fall away (t is finite or NaN), and w2's two halvings become one
+// of the sum: 11 FP64 operations for 27, the same bits.
 __device__ __forceinline__ void bspline_w64(double t, double* w)
 {
-    double t3 = t * t * t, t2 = t * t;
-    w[0] = (-1.0 / 6.0) * t3 + (3.0 / 6.0) * t2 + (-3.0 / 6.0) * t + (1.0 / 6.0);
-    w[1] = (3.0 / 6.0) * t3 + (-6.0 / 6.0) * t2 + (0.0 / 6.0) * t + (4.0 / 6.0);
-    w[2] = (-3.0 / 6.0) * t3 + (3.0 / 6.0) * t2 + (3.0 / 6.0) * t + (1.0 / 6.0);
-    w[3] = (1.0 / 6.0) * t3 + (0.0 / 6.0) * t2 + (0.0 / 6.0) * t + (0.0 / 6.0);
+    const double t2 = t * t, t3 = t2 * t, s3 = (1.0 / 6.0) * t3;
+    w[0] = __fma_rn(-0.5, t, __fma_rn(0.5, t2, -s3)) + 1.0 / 6.0;
+    w[1] = __fma_rn(0.5, t3, -t2) + 4.0 / 6.0;
+    w[2] = __fma_rn(0.5, (t2 - t3) + t, 1.0 / 6.0);
+    w[3] = s3;
 }
 
 // derivative of the basis with respect to the offset t
@@ -88,18 +98,34 @@ __device__ __forceinline__ void bspline_dw64(double t, double* w)
     w[3] = (3.0 / 6.0) * t2 + (0.0 / 6.0) * t + (0.0 / 6.0);
 }
 
-// Cell index and fractional offset along axis d of a coordinate on or inside
-// [a, b]; a NaN coordinate takes cell 0 (and a NaN offset).
-__device__ __forceinline__ int spline_locate64(const SplineGrid& g, int d, double x, double* t)
+// Cell index and fractional offset along axis d of a coordinate x; dx = x - a.
+// A coordinate beyond the far end b sets *outside (it can only lie in the last
+// cell, so the other cells skip the compare); a NaN coordinate takes any cell
+// (and a NaN offset).  floor() runs beside the FP64 pipe; the cell index comes
+// from the bits of its result, where the conversions to int and back and the
+// two range compares took four FP64-pipe slots an axis.
+__device__ __forceinline__ int spline_locate64(const SplineGrid& g, int d, double x, double dx,
+                                               double* t, bool* outside)
 {
-    double u = (x - g.a[d]) * g.dinv[d];
+    const double u = dx * g.dinv[d];
     double fu = floor(u);
-    int i;
-    if (fu > (double)(g.n[d] - 2)) i = g.n[d] - 2;
-    else if (!(fu >= 0.0)) i = 0;
-    else i = (int)fu;
-    *t = u - (double)i;
-    return i;
+    if (__double_as_longlong(fu) >= __double_as_longlong(g.top[d])) {  // fu >= n - 2 >= 0, or NaN
+        if (x > g.b[d]) *outside = true;
+        fu = g.top[d];
+    }
+    *t = u - fu;
+    const unsigned long long k = (unsigned long long)__double_as_longlong(fu);
+    const int sh = 1075 - (int)((k >> 52) & 0x7ff);  // fu = m 2^-sh, m its 53-bit significand
+    const unsigned long long m = (k & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    const int i = sh > 52 ? 0 : (int)(m >> (sh & 63));
+    return min(max(i, 0), g.n[d] - 2);
+}
+
+// x < a by dx = x - a, whose sign is exact: a negative number, not -0, not NaN
+__device__ __forceinline__ bool negative64(double dx)
+{
+    return (unsigned long long)__double_as_longlong(dx) - 0x8000000000000001ull <
+           0x7ff0000000000000ull;
 }
 
 // sum_a w0[a] sum_b w1[b] sum_c w2[c] C[it+a, ix+b, iy+c] of the interleaved
@@ -109,10 +135,12 @@ __device__ __forceinline__ void spline_sum_uv64(const SplineGrid& g, const doubl
                                                 const double* w1, const double* w2, double* u,
                                                 double* v)
 {
-    double au = 0.0, av = 0.0;
+    // the sums start at 0: their first terms are FMAs with 0 (one rounding, the
+    // product's), the others round product and sum separately
+    double au, av;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        double su = 0.0, sv = 0.0;
+        double su, sv;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const size_t e = (size_t)(it + a) * g.st + (size_t)(ix + b) * g.sx + iy;
@@ -127,11 +155,11 @@ __device__ __forceinline__ void spline_sum_uv64(const SplineGrid& g, const doubl
             }
             double bu = w2[0] * r0.x + w2[1] * r1.x + w2[2] * r2.x + w2[3] * r3.x;
             double bv = w2[0] * r0.y + w2[1] * r1.y + w2[2] * r2.y + w2[3] * r3.y;
-            su += w1[b] * bu;
-            sv += w1[b] * bv;
+            su = b == 0 ? __fma_rn(w1[0], bu, 0.0) : su + w1[b] * bu;
+            sv = b == 0 ? __fma_rn(w1[0], bv, 0.0) : sv + w1[b] * bv;
         }
-        au += w0[a] * su;
-        av += w0[a] * sv;
+        au = a == 0 ? __fma_rn(w0[0], su, 0.0) : au + w0[a] * su;
+        av = a == 0 ? __fma_rn(w0[0], sv, 0.0) : av + w0[a] * sv;
     }
     *u = au;
     *v = av;
@@ -150,23 +178,26 @@ __device__ __forceinline__ void spline_eval_uv64(const SplineGrid& g, const doub
                                                  double t, double x, double y, double* u,
                                                  double* v)
 {
-    if (XM == 0 && (t < g.a[0] || t > g.b[0] || x < g.a[1] || x > g.b[1] || y < g.a[2] ||
-                    y > g.b[2])) {
-        *u = 0.0;
-        *v = 0.0;
-        return;
-    }
     const double vv[3] = {t, x, y};
     double dl[3], f[3], w[3][4];
     int i[3];
+    bool out = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         double cl = vv[d];
         if (XM != 0) cl = vv[d] < g.a[d] ? g.a[d] : (vv[d] > g.b[d] ? g.b[d] : vv[d]);
-        dl[d] = vv[d] - cl;
-        i[d] = spline_locate64(g, d, cl, &f[d]);
-        bspline_w64(f[d], w[d]);
+        const double dx = cl - g.a[d];
+        if (XM != 0) dl[d] = vv[d] - cl;
+        else if (negative64(dx)) out = true;
+        i[d] = spline_locate64(g, d, cl, dx, &f[d], &out);
     }
+    if (XM == 0 && out) {
+        *u = 0.0;
+        *v = 0.0;
+        return;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) bspline_w64(f[d], w[d]);
     double au, av;
     spline_sum_uv64(g, c, i[0], i[1], i[2], w[0], w[1], w[2], &au, &av);
     if (XM == 2) {
@@ -200,7 +231,7 @@ struct FlowSpline64 {
         double tt = p[0] * t;
         double u, v;
         if (SPH == 1 || SPH == 2) {
-            double xx = SPH == 1 ? py_fmod(y[0] - 180.0, 360.0) - 180.0 : py_fmod(y[0], 360.0);
+            double xx = SPH == 1 ? py_mod360(y[0] - 180.0) - 180.0 : py_mod360(y[0]);
             double yy = y[1];
             spline_eval_uv64<XM>(g, c, tt, xx, yy, &u, &v);
             dy[0] = p[0] * u * 180.0 / (NBCS_PI * r * nbcs_cos_deg(yy));

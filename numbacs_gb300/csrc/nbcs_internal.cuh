@@ -87,6 +87,7 @@ struct Params {
 // (n-1)/(b-a) precomputed on the host exactly as the device would.
 struct SplineGrid {
     double a[3], b[3], dinv[3];
+    double top[3];  // n - 2, the last cell
     int n[3];
     int sx, st;  // node strides of the (nt+2, nx+2, ny+2) coefficient block
 };
@@ -99,6 +100,7 @@ inline SplineGrid make_grid(const double* g)
         s.b[d] = g[3 * d + 1];
         s.n[d] = (int)g[3 * d + 2];
         s.dinv[d] = (double)(s.n[d] - 1) / (s.b[d] - s.a[d]);
+        s.top[d] = (double)(s.n[d] - 2);
     }
     s.sx = s.n[2] + 2;
     s.st = (s.n[1] + 2) * (s.n[2] + 2);
