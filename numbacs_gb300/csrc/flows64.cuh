@@ -12,6 +12,7 @@
 #pragma once
 
 #include "detmath.h"
+#include "intfp64.h"
 #include "nbcs_internal.cuh"
 
 namespace nbcs {
@@ -66,7 +67,7 @@ __device__ __forceinline__ double py_mod360(double a)
     double m = a;
     if ((hi & 0x7fffffffu) >= 0x40768000u) m = fmod(a, 360.0);  // |a| >= 360, inf, NaN
     const long long mb = __double_as_longlong(m);
-    if ((mb & 0x7fffffffffffffffll) == 0) return 0.0;
+    if (ip_zero(m)) return 0.0;
     return mb < 0 ? m + 360.0 : m;  // NaN stays NaN
 }
 

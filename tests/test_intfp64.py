@@ -1,0 +1,114 @@
+"""IEEE double operations on the integer pipe (csrc/intfp64.h), compiled for the
+host and checked against the host's own FP64 arithmetic: products, quotients
+and roots bit for bit, logarithms and reciprocal roots to a fraction of an ulp.
+The FP32 estimates that the device takes from its special-function unit are off
+by up to 2^-22; the host's are moved by up to three FP32 ulps either way."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SRC = r"""
+#include "intfp64.h"
+extern "C" {
+void t_mul(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_mul(a[i], b[i]); }
+void t_div(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_div(a[i], ip_reciprocal(b[i])); }
+void t_sqrt(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_sqrt(a[i]); }
+void t_log(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_log(a[i]); }
+void t_rsqrt(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_apply_fit(b[i], ip_rsqrt_fit(a[i])); }
+}
+"""
+
+
+@pytest.fixture(scope="module", params=[0, -3, 3])
+def lib(request, tmp_path_factory):
+    d = tmp_path_factory.mktemp("intfp64")
+    src, out = d / "t.cpp", d / "t.so"
+    src.write_text(SRC)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-ffp-contract=off",
+                    "-DNBCS_INTFP64_ESTIMATE_ULPS=(%d)" % request.param,
+                    "-I", os.path.join(ROOT, "numbacs_gb300", "csrc"), str(src), "-o", str(out)],
+                   check=True)
+    return ctypes.CDLL(str(out))
+
+
+def _call(lib, name, a, b):
+    o = np.empty_like(a)
+    p = ctypes.POINTER(ctypes.c_double)
+    getattr(lib, name)(a.ctypes.data_as(p), b.ctypes.data_as(p), ctypes.c_long(len(a)),
+                       o.ctypes.data_as(p))
+    return o
+
+
+def _bits(a):
+    return a.view(np.uint64)
+
+
+def _numbers(rng, n, lo, hi):
+    """Doubles of exponents [lo, hi): a part with short significands, all ones
+    or a single one, where quotients and roots come out exact or next to it."""
+    m = rng.integers(0, 1 << 52, n, dtype=np.uint64)
+    k = rng.integers(0, 8, n)
+    m[k == 0] = 0
+    m[k == 1] = (1 << 52) - 1
+    cut = rng.integers(1, 52, n, dtype=np.uint64)
+    low = (np.uint64(1) << cut) - np.uint64(1)
+    m = np.where(k == 2, m & ~low, m)
+    m = np.where(k == 3, m | low, m)
+    m = np.where(k == 4, m & np.uint64(15), m)
+    e = (rng.integers(lo, hi, n) + 1023).astype(np.uint64)
+    s = rng.integers(0, 2, n, dtype=np.uint64)
+    return ((s << np.uint64(63)) | (e << np.uint64(52)) | m).view(np.float64)
+
+
+EDGES = np.array([0.0, -0.0, 5e-324, 2.2250738585072014e-308, 2.0 ** -256, 2.0 ** -255, 2.0 ** 255,
+                  np.nextafter(2.0 ** 256, 0), 2.0 ** 256, 1.7976931348623157e308, np.inf, -np.inf,
+                  np.nan, 1.0, np.nextafter(1.0, 0), np.nextafter(1.0, 2), 2.0, 3.0, -1.0 / 3.0])
+
+
+def _pairs(span):
+    rng = np.random.default_rng(5)
+    a, b = _numbers(rng, 200000, -span, span), _numbers(rng, 200000, -span, span)
+    g = np.meshgrid(EDGES, EDGES, indexing="ij")
+    return (np.concatenate([a, a * b, g[0].ravel()]), np.concatenate([b, b, g[1].ravel()]))
+
+
+@pytest.mark.parametrize("span", [2, 120, 255])
+def test_products_quotients_roots_bit_for_bit(lib, span):
+    a, b = _pairs(span)
+    with np.errstate(all="ignore"):
+        for name, want in (("t_mul", a * b), ("t_div", a / b)):
+            got = _call(lib, name, a, b)
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan), name
+            assert np.array_equal(_bits(got)[~nan], _bits(want)[~nan]), name
+        for x in (a, a * a, np.nextafter(a * a, np.inf)):
+            want, got = np.sqrt(x), _call(lib, "t_sqrt", x, x)
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan)
+            assert np.array_equal(_bits(got)[~nan], _bits(want)[~nan])
+
+
+def _ulps(got, want):
+    """|got - want| in ulps of want (a long double)."""
+    ulp = np.ldexp(1.0, np.frexp(want.astype(np.float64))[1] - 53)
+    return np.abs(got.astype(np.longdouble) - want) / ulp
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).nmant < 63, reason="needs an 80-bit long double")
+def test_logarithm_and_reciprocal_root(lib):
+    rng = np.random.default_rng(6)
+    x = np.concatenate([1.0 + rng.random(100000) * s for s in (1e-12, 0.01, 1.0)] +
+                       [np.exp(rng.random(100000) * 160.0), 1.0 + np.arange(1, 513) / 256.0,
+                        [np.nextafter(1.0, 2), np.nextafter(2.0, 1), 2.0, np.nextafter(2.0 ** 256, 0),
+                         2.0 ** 256, 1e300]])
+    # half an ulp of rounding, 2^-60 relative of fixed point and series
+    assert _ulps(_call(lib, "t_log", x, x), np.log(x.astype(np.longdouble))).max() < 0.55
+    a = np.abs(_numbers(rng, 200000, -200, 200))
+    b = _numbers(rng, 200000, -200, 200)
+    want = b.astype(np.longdouble) / np.sqrt(a.astype(np.longdouble))
+    assert _ulps(_call(lib, "t_rsqrt", a, b), want).max() < 0.55
