@@ -101,6 +101,11 @@ const char* nbcs_last_error(void);
 size_t nbcs_spline_prefilter_scratch_bytes(int32_t nt, int32_t nx, int32_t ny);
 int nbcs_spline_prefilter_3d(const double* f, int32_t nt, int32_t nx, int32_t ny,
                              double* coef, void* scratch, size_t scratch_bytes, void* stream);
+/* The same of the two velocity components at once, in the launches of one:
+ * scratch >= 2 * nbcs_spline_prefilter_scratch_bytes(). */
+int nbcs_spline_prefilter_uv(const double* u, const double* v, int32_t nt, int32_t nx, int32_t ny,
+                             double* coef_u, double* coef_v, void* scratch, size_t scratch_bytes,
+                             void* stream);
 
 /* get_flow_2D coefficient capture (flows.py:156-254 closes over C_eval_u /
  * C_eval_v): interleave cu, cv (n nodes each) into coef_uv (2n doubles) and,

@@ -78,6 +78,8 @@ SIGNATURES = {
     "nbcs_last_error": (ctypes.c_char_p, []),
     "nbcs_spline_prefilter_scratch_bytes": (_sz, [_i32, _i32, _i32]),
     "nbcs_spline_prefilter_3d": (ctypes.c_int, [_vp, _i32, _i32, _i32, _vp, _vp, _sz, _vp]),
+    "nbcs_spline_prefilter_uv": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp, _sz,
+                                                _vp]),
     "nbcs_spline_pack_uv": (ctypes.c_int, [_vp, _vp, _i64, _vp, _vp, _vp]),
     "nbcs_eval_rhs": (ctypes.c_int, [_FP, _vp, _i32, _vp, _i64, _vp, _i32, _vp]),
     "nbcs_flowmap_grid_2d": (ctypes.c_int, [_FP, _d, _d, _vp, _i32, _vp, _i32, _vp, _i32, _d, _d,

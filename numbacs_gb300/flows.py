@@ -143,8 +143,12 @@ def get_interp_arrays_2D(tvals, xvals, yvals, U, V):
     yv = np.asarray(yvals.cpu() if isinstance(yvals, torch.Tensor) else yvals, dtype=np.float64)
     grid_vel = ((float(tv[0]), float(tv[-1]), nt), (float(xv[0]), float(xv[-1]), nx),
                 (float(yv[0]), float(yv[-1]), ny))
-    Cu = _prefilter(Ud)
-    Cv = _prefilter(Vd)
+    L = _lib.load()
+    Cu, Cv = D.empty((nt + 2, nx + 2, ny + 2)), D.empty((nt + 2, nx + 2, ny + 2))
+    nbytes = 2 * L.nbcs_spline_prefilter_scratch_bytes(nt, nx, ny)
+    scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=Ud.device)
+    _lib.check(L.nbcs_spline_prefilter_uv(D.ptr(Ud), D.ptr(Vd), nt, nx, ny, D.ptr(Cu), D.ptr(Cv),
+                                          D.ptr(scratch), nbytes, D.stream_ptr()))
     return grid_vel, D.finish(Cu, as_torch), D.finish(Cv, as_torch)
 
 
