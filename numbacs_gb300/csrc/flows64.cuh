@@ -129,17 +129,50 @@ __device__ __forceinline__ bool negative64(double dx)
            0x7ff0000000000000ull;
 }
 
+// One stencil row: w[0] r0 + w[1] r1 + w[2] r2 + w[3] r3 of both components,
+// every product and sum rounded as the reference rounds it.  FIT: the products
+// on the integer pipe (intfp64.h, the same bits).
+template <bool FIT>
+__device__ __forceinline__ double2 row_dot64(const double* w, double2 r0, double2 r1, double2 r2,
+                                             double2 r3)
+{
+    auto mul = [](double a, double b) { return FIT ? ip_mul_fit(a, b) : a * b; };
+    return make_double2(mul(w[0], r0.x) + mul(w[1], r1.x) + mul(w[2], r2.x) + mul(w[3], r3.x),
+                        mul(w[0], r0.y) + mul(w[1], r1.y) + mul(w[2], r2.y) + mul(w[3], r3.y));
+}
+
+// every one of four doubles is in the range of the integer products
+__device__ __forceinline__ bool fit4(double a, double b, double c, double d)
+{
+    return ((((unsigned)__double2hiint(a) - 0x30000000u) |
+             ((unsigned)__double2hiint(b) - 0x30000000u) |
+             ((unsigned)__double2hiint(c) - 0x30000000u) |
+             ((unsigned)__double2hiint(d) - 0x30000000u)) & 0x60000000u) == 0;
+}
+
+// the first term of a sum that starts at 0 (one rounding, the product's), and a
+// further one
+__device__ __forceinline__ double first64(double w, double b)
+{
+    return ip_fits(ip_bits(w), ip_bits(b)) ? ip_mul_fit(w, b) : __fma_rn(w, b, 0.0);
+}
+__device__ __forceinline__ double next64(double s, double w, double b) { return s + ip_mul(w, b); }
+
 // sum_a w0[a] sum_b w1[b] sum_c w2[c] C[it+a, ix+b, iy+c] of the interleaved
-// (u, v) coefficient block
+// (u, v) coefficient block.  The 168 products of a point went to the FP64 pipe
+// beside its 126 sums, at 19 cycles of the SM each; on the integer pipe they
+// take 11.  Rows or weights out of the integer arithmetic's range (zeros above
+// all: velocity masked over land, a point on a grid node) take the FP64 pipe.
+// The time levels are a rolled loop: unrolled, the sixteen rows of integer code
+// outgrow the instruction caches.
 __device__ __forceinline__ void spline_sum_uv64(const SplineGrid& g, const double2* __restrict__ c,
                                                 int it, int ix, int iy, const double* w0,
                                                 const double* w1, const double* w2, double* u,
                                                 double* v)
 {
-    // the sums start at 0: their first terms are FMAs with 0 (one rounding, the
-    // product's), the others round product and sum separately
-    double au, av;
-#pragma unroll
+    const bool wfit = fit4(w2[0], w2[1], w2[2], w2[3]);
+    double au = 0.0, av = 0.0;
+#pragma unroll 1
     for (int a = 0; a < 4; ++a) {
         double su, sv;
 #pragma unroll
@@ -154,13 +187,15 @@ __device__ __forceinline__ void spline_sum_uv64(const SplineGrid& g, const doubl
                 r2 = __ldg(row + 2);
                 r3 = __ldg(row + 3);
             }
-            double bu = w2[0] * r0.x + w2[1] * r1.x + w2[2] * r2.x + w2[3] * r3.x;
-            double bv = w2[0] * r0.y + w2[1] * r1.y + w2[2] * r2.y + w2[3] * r3.y;
-            su = b == 0 ? __fma_rn(w1[0], bu, 0.0) : su + w1[b] * bu;
-            sv = b == 0 ? __fma_rn(w1[0], bv, 0.0) : sv + w1[b] * bv;
+            const bool fit = wfit && fit4(r0.x, r1.x, r2.x, r3.x) && fit4(r0.y, r1.y, r2.y, r3.y);
+            const double2 d = fit ? row_dot64<true>(w2, r0, r1, r2, r3)
+                                  : row_dot64<false>(w2, r0, r1, r2, r3);
+            su = b == 0 ? first64(w1[0], d.x) : next64(su, w1[b], d.x);
+            sv = b == 0 ? first64(w1[0], d.y) : next64(sv, w1[b], d.y);
         }
-        au = a == 0 ? __fma_rn(w0[0], su, 0.0) : au + w0[a] * su;
-        av = a == 0 ? __fma_rn(w0[0], sv, 0.0) : av + w0[a] * sv;
+        const double wa = a == 0 ? w0[0] : a == 1 ? w0[1] : a == 2 ? w0[2] : w0[3];
+        au = a == 0 ? first64(wa, su) : next64(au, wa, su);
+        av = a == 0 ? first64(wa, sv) : next64(av, wa, sv);
     }
     *u = au;
     *v = av;
