@@ -13,9 +13,9 @@ __global__ void __launch_bounds__(kBatchThreads)
 batch64_kernel(BatchHeader* hdr, const DevFlow64* __restrict__ flows,
                const DevField* __restrict__ fields, int nfields, int nmax)
 {
-    __shared__ double2 ks[12 * kThreads64];
-    double2* kc = ks + threadIdx.x;
-    const int lane = threadIdx.x & 31;
+    __shared__ double ks[12 * kThreads64];
+    double* kc = ks + threadIdx.x;
+    const int lane = threadIdx.x & 31, q = lane & 1;
     const long long total = hdr->total_chunks;
     for (;;) {
         unsigned long long c = 0ull;
@@ -24,39 +24,43 @@ batch64_kernel(BatchHeader* hdr, const DevFlow64* __restrict__ flows,
         if ((long long)c >= total) break;
         const int f = batch_find<kByChunk>(fields, nfields, (long long)c);
         const DevField& F = fields[f];
-        int i, j;
-        if (!batch_particle(F, (long long)c, lane, &i, &j)) continue;
-        const long p = (long)i * F.ny + j;
-        double yv[2] = {0.0, 0.0};
-        int st = NBCS_PARTICLE_MASKED;
-        Dop853Stats s = {0, 0, 0};
-        if (!(F.mask && F.mask[p])) {
-            yv[0] = F.x[i];
-            yv[1] = F.y[j];
-            const DevFlow64& fl = flows[F.flow];
-            switch (fl.kind) {
-            case NBCS_FLOW_DOUBLE_GYRE:
-                st = dop853_solve64(FlowDG64{}, F.P, F.ts, F.te, yv, F.rtol, F.atol, nmax, kc, &s);
-                break;
-            case NBCS_FLOW_BICKLEY:
-                st = dop853_solve64(FlowBickley64{}, F.P, F.ts, F.te, yv, F.rtol, F.atol, nmax, kc,
-                                    &s);
-                break;
-            default:
-                if (fl.spherical == 1)
-                    st = dop853_solve64(FlowSpline64<1>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te, yv,
-                                        F.rtol, F.atol, nmax, kc, &s);
-                else if (fl.spherical == 2)
-                    st = dop853_solve64(FlowSpline64<2>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te, yv,
-                                        F.rtol, F.atol, nmax, kc, &s);
-                else
-                    st = dop853_solve64(FlowSpline64<0>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te, yv,
-                                        F.rtol, F.atol, nmax, kc, &s);
-                break;
+        // a chunk of 32 particles in two halves (of 16: spline fields, whose plan
+        // counts two lanes a particle), two lanes a particle here
+        for (int half = 0; half < 2 / F.lp; ++half) {
+            int i, j;
+            if (!batch_particle_of(F, (long long)c, half * 16 + (lane >> 1), &i, &j)) continue;
+            const long p = (long)i * F.ny + j;
+            double yv = 0.0;
+            int st = NBCS_PARTICLE_MASKED;
+            Dop853Stats s = {0, 0, 0};
+            if (!(F.mask && F.mask[p])) {
+                yv = q ? F.y[j] : F.x[i];
+                const DevFlow64& fl = flows[F.flow];
+                switch (fl.kind) {
+                case NBCS_FLOW_DOUBLE_GYRE:
+                    st = dop853_solve64(FlowDG64<>{}, F.P, F.ts, F.te, &yv, q, F.rtol, F.atol, nmax,
+                                        kc, &s);
+                    break;
+                case NBCS_FLOW_BICKLEY:
+                    st = dop853_solve64(FlowBickley64{}, F.P, F.ts, F.te, &yv, q, F.rtol, F.atol,
+                                        nmax, kc, &s);
+                    break;
+                default:
+                    if (fl.spherical == 1)
+                        st = dop853_solve64(FlowSpline64<1>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te,
+                                            &yv, q, F.rtol, F.atol, nmax, kc, &s);
+                    else if (fl.spherical == 2)
+                        st = dop853_solve64(FlowSpline64<2>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te,
+                                            &yv, q, F.rtol, F.atol, nmax, kc, &s);
+                    else
+                        st = dop853_solve64(FlowSpline64<0>{fl.g, fl.c, fl.r}, F.P, F.ts, F.te,
+                                            &yv, q, F.rtol, F.atol, nmax, kc, &s);
+                    break;
+                }
             }
+            F.out[2 * p + q] = yv;
+            if (F.status && !q) F.status[p] = st;
         }
-        reinterpret_cast<double2*>(F.out)[p] = make_double2(yv[0], yv[1]);
-        if (F.status) F.status[p] = st;
     }
 }
 

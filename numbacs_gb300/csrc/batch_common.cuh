@@ -91,19 +91,25 @@ __device__ __forceinline__ int batch_find(const DevField* __restrict__ fields, i
     return lo;
 }
 
-// Particle (i, j) of lane `lane` in work unit c of field F; false past the grid edge.
-__device__ __forceinline__ bool batch_particle(const DevField& F, long long c, int lane, int* i,
-                                               int* j)
+// Particle (i, j) number p of work unit c of field F; false past the grid edge.
+__device__ __forceinline__ bool batch_particle_of(const DevField& F, long long c, int p, int* i,
+                                                  int* j)
 {
-    const int lp = F.lp, tj = batch_tile_j(lp);
+    const int tj = batch_tile_j(F.lp);
     const long r = (long)(c - F.chunk0);
     const int tiles_j = (F.ny + tj - 1) / tj;
     const long tI = r / tiles_j;
     const int tJ = (int)(r - tI * tiles_j);
-    const int p = lane / lp;
     *i = (int)(tI * kBatchTileI) + p / tj;
     *j = tJ * tj + p % tj;
     return *i < F.nx && *j < F.ny;
+}
+
+// the particle of lane `lane` at the field's lanes a particle
+__device__ __forceinline__ bool batch_particle(const DevField& F, long long c, int lane, int* i,
+                                               int* j)
+{
+    return batch_particle_of(F, c, lane / F.lp, i, j);
 }
 
 int launch_batch32_tiles(const DevFlow32* flows, const DevField* fields, int nfields,

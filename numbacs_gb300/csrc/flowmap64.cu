@@ -1,7 +1,7 @@
 // FP64 flow-map integration (the plain path) and the RHS probe entry point.
 //
 // Replaces flowmap_grid_2D (integration.py:123-182) with method="dop853":
-// one thread per particle runs the FP64 DOP853 solver of dop853_64.cuh on a
+// two lanes per particle run the FP64 DOP853 solver of dop853_64.cuh on a
 // device-compiled right-hand side.  Compiled with -fmad=false.  The particle
 // <-> thread map does not enter the arithmetic: results are the oracle's bit
 // for bit whatever the tile shape.
@@ -11,43 +11,48 @@
 
 namespace nbcs {
 
-// One warp per block, a 4 x 8 tile of particles.  The kernel is bound by the
-// FP64 pipe, which two or three warps a partition keep busy, so what counts is
-// an even share of the work: single-warp blocks are the finest unit that the
-// SMs can take from the launch.  Against 256-thread blocks (32 x 8 tiles), with
-// the operations that left the FP64 pipe in the same change: double gyre 401 x
-// 201 8.09 -> 5.45 ms, geophysical flow 338 x 126 (rtol 1e-6) 56.7 -> 31.3 ms
-// (176 blocks had kept the SMs busy 56 % of the time), 21 x 11 double gyre
-// 1.74 -> 1.02 ms.
+// One warp per block, a 4 x 4 tile of particles at two lanes each.  The kernel
+// is bound by the FP64 pipe, which a few warps a partition keep busy, so what
+// counts is an even share of the work: single-warp blocks are the finest unit
+// that the SMs can take from the launch (256-thread blocks of one lane a
+// particle kept them busy 56 % of the time on a 338 x 126 grid).
 constexpr int kFm64Block = 32;
 
-template <class Flow>
-__global__ void __launch_bounds__(kFm64Block)
+// Registers for 20 warps an SM (96 a thread): 22.1 ms for the geophysical flow
+// map of 338 x 126 particles, 22.8 and 24.0 ms with 16 and 12 warps and no
+// spills.
+constexpr int kFm64MinBlocks = 20;
+
+template <class Flow, bool FEW>
+__global__ void __launch_bounds__(kFm64Block, kFm64MinBlocks)
 flowmap64_kernel(Flow fl, Params P, double ts, double te, const double* __restrict__ x,
                  const double* __restrict__ y, int nx, int nyv, AuxGrid aux,
                  const uint8_t* __restrict__ mask, double* __restrict__ out,
                  int32_t* __restrict__ status, int32_t* __restrict__ stats, double rtol,
                  double atol, int nmax)
 {
-    __shared__ double2 ks[12 * kFm64Block];
-    double2* kc = ks + threadIdx.x;
-    using S = TileShape<1, kFm64Block>;
+    __shared__ double ks[12 * kFm64Block];
+    double* kc = ks + threadIdx.x;
+    const int q = threadIdx.x & 1;
+    using S = TileShape<2, kFm64Block>;
     const long nthreads = (long)((nx + S::TI - 1) / S::TI) * ((nyv + S::TJ - 1) / S::TJ) * kFm64Block;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < nthreads;
          t += (long)gridDim.x * blockDim.x) {
         int i, j;
-        if (!tile_particle<1, kFm64Block>(t, nx, nyv, &i, &j)) continue;
+        // the lanes of a pair share the particle: they leave together
+        if (!tile_particle<2, kFm64Block>(t, nx, nyv, &i, &j)) continue;
         const long k = (long)i * nyv + j;
         if (!particle_exists(aux, k)) continue;
-        double yv[2] = {0.0, 0.0}, x0, y0;
+        double yv = 0.0, x0, y0;
         int st = NBCS_PARTICLE_MASKED;
         Dop853Stats s = {0, 0, 0};
         if (particle_start(aux, x, y, mask, nx, i, j, &x0, &y0)) {
-            yv[0] = x0;
-            yv[1] = y0;
-            st = dop853_solve64<Flow, kFm64Block>(fl, P, ts, te, yv, rtol, atol, nmax, kc, &s);
+            yv = q ? y0 : x0;
+            st = dop853_solve64<Flow, kFm64Block, false, FEW>(fl, P, ts, te, &yv, q, rtol, atol, nmax,
+                                                              kc, &s);
         }
-        reinterpret_cast<double2*>(out)[k] = make_double2(yv[0], yv[1]);
+        out[2 * k + q] = yv;
+        if (q) continue;
         if (status) status[k] = st;
         if (stats) {
             stats[3 * k] = s.accepted;
@@ -61,12 +66,11 @@ template <class Flow>
 __global__ void rhs64_kernel(Flow fl, Params P, const double* __restrict__ ty, long n,
                              double* __restrict__ dy)
 {
-    for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += (long)gridDim.x * blockDim.x) {
-        double yv[2] = {ty[3 * k + 1], ty[3 * k + 2]}, d[2];
-        fl(ty[3 * k], yv, d, P);
-        dy[2 * k] = d[0];
-        dy[2 * k + 1] = d[1];
+    const int q = threadIdx.x & 1;
+    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * n;
+         t += (long)gridDim.x * blockDim.x) {
+        const long k = t >> 1;
+        dy[2 * k + q] = fl(ty[3 * k], ty[3 * k + 1 + q], q, P);
     }
 }
 
@@ -75,7 +79,24 @@ struct Launch64 {
     template <class Flow>
     int operator()(const Flow& fl) const
     {
-        using S = TileShape<1, kFm64Block>;
+        return run<Flow, false>(fl);
+    }
+    // An analytic flow on fewer warps than the SMs have partitions (each then
+    // has its own): 21 x 11 double gyre 770 -> 622 us.
+    int operator()(const FlowDG64<>& fl) const
+    {
+        return few() ? run<FlowDG64<true>, true>(FlowDG64<true>{}) : run<FlowDG64<>, false>(fl);
+    }
+    bool few() const
+    {
+        using S = TileShape<2, kFm64Block>;
+        return (long)((a->nx + S::TI - 1) / S::TI) * ((a->nyv() + S::TJ - 1) / S::TJ) <=
+               4L * sm_count();
+    }
+    template <class Flow, bool FEW>
+    int run(const Flow& fl) const
+    {
+        using S = TileShape<2, kFm64Block>;
         const int threads = kFm64Block;
         long blocks = (long)((a->nx + S::TI - 1) / S::TI) * ((a->nyv() + S::TJ - 1) / S::TJ);
         if (a->blocks_per_sm > 0) {
@@ -83,7 +104,7 @@ struct Launch64 {
             if (blocks > cap) blocks = cap;
         }
         if (blocks > (1L << 30)) blocks = 1L << 30;
-        flowmap64_kernel<<<(unsigned)blocks, threads, 0, a->stream>>>(
+        flowmap64_kernel<Flow, FEW><<<(unsigned)blocks, threads, 0, a->stream>>>(
             fl, a->P, a->ts, a->te, a->x, a->y, a->nx, a->nyv(), a->aux, a->mask, a->out,
             a->status, a->stats, a->rtol, a->atol, a->nmax);
         NBCS_LAUNCH_CHECK();
@@ -91,33 +112,33 @@ struct Launch64 {
     }
 };
 
-// flowmap_n / flowmap_n_grid_2D (integration.py:65-121, :468-534): one thread
+// flowmap_n / flowmap_n_grid_2D (integration.py:65-121, :468-534): two lanes
 // per point of a list, the positions at the n output times teval by dense
-// output of one DOP853 run (16 stage slots per thread); masked points and the
-// outputs past a failure stay 0.
+// output of one DOP853 run; masked points and the outputs past a failure stay 0.
 constexpr int kDense64Block = 32;
 
 template <class Flow>
 __global__ void __launch_bounds__(kDense64Block)
 flowmap64_n_kernel(Flow fl, Params P, const double* __restrict__ pts, long npts,
                    const double* __restrict__ teval, int n, const uint8_t* __restrict__ mask,
-                   double2* __restrict__ out, int32_t* __restrict__ status, double rtol,
+                   double* __restrict__ out, int32_t* __restrict__ status, double rtol,
                    double atol, int nmax)
 {
-    __shared__ double2 ks[16 * kDense64Block];
-    double2* kc = ks + threadIdx.x;
-    const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double ks[16 * kDense64Block];
+    double* kc = ks + threadIdx.x;
+    const int q = threadIdx.x & 1;
+    const long k = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
     if (k >= npts) return;
-    double2* o = out + k * n;
-    for (int m = 0; m < n; ++m) o[m] = make_double2(0.0, 0.0);
+    double* o = out + 2 * k * n + q;
+    for (int m = 0; m < n; ++m) o[2 * m] = 0.0;
     int st = NBCS_PARTICLE_MASKED;
     if (!(mask && mask[k])) {
-        double yv[2] = {pts[2 * k], pts[2 * k + 1]};
+        double yv = pts[2 * k + q];
         Dop853Stats s;
-        st = dop853_solve64<Flow, kDense64Block, true>(fl, P, teval[0], teval[n - 1], yv, rtol,
+        st = dop853_solve64<Flow, kDense64Block, true>(fl, P, teval[0], teval[n - 1], &yv, q, rtol,
                                                        atol, nmax, kc, &s, teval, n, o);
     }
-    if (status) status[k] = st;
+    if (status && !q) status[k] = st;
 }
 
 struct LaunchDense64 {
@@ -135,10 +156,9 @@ struct LaunchDense64 {
     template <class Flow>
     int operator()(const Flow& fl) const
     {
-        const long blocks = (npts + kDense64Block - 1) / kDense64Block;
+        const long blocks = (2 * npts + kDense64Block - 1) / kDense64Block;
         flowmap64_n_kernel<<<(unsigned)blocks, kDense64Block, 0, stream>>>(
-            fl, P, pts, npts, teval, n, mask, reinterpret_cast<double2*>(out), status, rtol, atol,
-            nmax);
+            fl, P, pts, npts, teval, n, mask, out, status, rtol, atol, nmax);
         NBCS_LAUNCH_CHECK();
         return NBCS_OK;
     }
@@ -154,7 +174,8 @@ struct LaunchRhs64 {
     int operator()(const Flow& fl) const
     {
         int threads = 128;
-        long blocks = (n + threads - 1) / threads;
+        long blocks = (2 * n + threads - 1) / threads;
+        if (blocks > (1L << 30)) blocks = 1L << 30;
         if (blocks < 1) blocks = 1;
         rhs64_kernel<<<(unsigned)blocks, threads, 0, stream>>>(fl, P, ty, n, dy);
         NBCS_LAUNCH_CHECK();
@@ -166,7 +187,7 @@ template <class F>
 static int dispatch64(const nbcs_flow* flow, const F& f)
 {
     switch (flow->kind) {
-    case NBCS_FLOW_DOUBLE_GYRE: return f(FlowDG64{});
+    case NBCS_FLOW_DOUBLE_GYRE: return f(FlowDG64<>{});
     case NBCS_FLOW_BICKLEY: return f(FlowBickley64{});
     default: {
         SplineGrid g = make_grid(flow->grid);

@@ -11,50 +11,67 @@
 //   spline RHS    flows.py:154-254 (interpolation.eval_spline, k=3)
 #pragma once
 
-#include "detmath.h"
-#include "intfp64.h"
+#include "dop853_64.cuh"
 #include "nbcs_internal.cuh"
 
 namespace nbcs {
 
 #define NBCS_PI 3.141592653589793
 
+// A right-hand side is called by the two lanes of a particle together, each
+// with its own component q of the position, and gives each its own component of
+// the velocity.
+// FEW: as in dop853_solve64, products on the FP64 pipe.
+template <bool FEW = false>
 struct FlowDG64 {
-    __device__ __forceinline__ void operator()(double t, const double* y, double* dy,
-                                               const Params& P) const
+    static __device__ __forceinline__ double mul(double a, double b)
+    {
+        return FEW ? a * b : ip_mul(a, b);
+    }
+    __device__ __forceinline__ double operator()(double t, double y, int q, const Params& P) const
     {
         const double* p = P.v;
-        double tt = p[0] * t;
-        double a = p[2] * sin(p[4] * tt + p[5]);
-        double b = 1.0 - 2.0 * a;
-        double f = a * (y[0] * y[0]) + b * y[0];
-        double df = 2.0 * a * y[0] + b;
-        double sf, cf, sy, cy;
-        sincos(NBCS_PI * f, &sf, &cf);
-        sincos(NBCS_PI * y[1], &sy, &cy);
-        dy[0] = p[0] * (-NBCS_PI * p[1] * sf * cy - p[3] * y[0]);
-        dy[1] = p[0] * (NBCS_PI * p[1] * cf * sy * df - p[3] * y[1]);
+        const double yo = other64(y), X = q ? yo : y, Y = q ? y : yo;
+        const double tt = p[0] * t;
+        // (products on the FP64 pipe too, as far as it has room beside the sines)
+        const double a = p[2] * ip_sin(p[4] * tt + p[5]);
+        const double a2 = 2.0 * a, b = 1.0 - a2;
+        const double f = mul(a, mul(X, X)) + mul(b, X);
+        const double df = mul(a2, X) + b;
+        // lane 0 takes sin, cos of pi f, lane 1 of pi Y
+        double s, c;
+        ip_sincos(NBCS_PI * (q ? Y : f), &s, &c);
+        const double co = other64(c);
+        // dx = -pi A sin(pi f) cos(pi Y), dy = pi A cos(pi f) sin(pi Y) df
+        const double w = (q ? NBCS_PI : -NBCS_PI) * p[1];
+        const double v = mul(mul(w, q ? co : s), q ? s : co);
+        return p[0] * (v * (q ? df : 1.0) - p[3] * y);
     }
 };
 
 struct FlowBickley64 {
-    __device__ __forceinline__ void operator()(double t, const double* y, double* dy,
-                                               const Params& P) const
+    __device__ __forceinline__ double operator()(double t, double y, int q, const Params& P) const
     {
         const double* p = P.v;
-        double tt = p[0] * t;
-        double Y = y[1] / p[2];
-        double ch = cosh(Y);
-        double sech2 = 1.0 / (ch * ch);
-        double s1 = y[0] - p[9] * tt, s2 = y[0] - p[10] * tt, s3 = y[0] - p[11] * tt;
-        double sn1, cs1, sn2, cs2, sn3, cs3;
-        sincos(p[6] * s1, &sn1, &cs1);
-        sincos(p[7] * s2, &sn2, &cs2);
-        sincos(p[8] * s3, &sn3, &cs3);
-        dy[0] = p[0] * (p[1] * sech2 + 2.0 * p[1] * tanh(Y) * sech2
-                                           * (p[3] * cs1 + p[4] * cs2 + p[5] * cs3));
-        dy[1] = -p[0] * (p[1] * p[2] * sech2
-                         * (p[3] * p[6] * sn1 + p[4] * p[7] * sn2 + p[5] * p[8] * sn3));
+        const double yo = other64(y), X = q ? yo : y, Yv = q ? y : yo;
+        const double tt = p[0] * t;
+        const double Y = ip_div(Yv, ip_reciprocal(p[2]));
+        const double ch = cosh(Y), th = tanh(Y);
+        const double sech2 = quot64(1.0, ip_mul(ch, ch));
+        // lane 0 takes the cosines, lane 1 the sines
+        double tr[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            double s, c;
+            ip_sincos(ip_mul(p[6 + k], X - ip_mul(p[9 + k], tt)), &s, &c);
+            tr[k] = q ? ip_mul(p[3 + k], p[6 + k]) : p[3 + k];
+            tr[k] = ip_mul(tr[k], q ? s : c);
+        }
+        const double sum = tr[0] + tr[1] + tr[2];
+        // dx = U sech^2 + 2 U tanh sech^2 (sum A cos), dy = -(U L sech^2 (sum A k sin))
+        const double us = ip_mul(q ? ip_mul(p[1], p[2]) : p[1], sech2);
+        const double r = ip_mul(q ? us : ip_mul(ip_mul(ip_scale(p[1], 1), th), sech2), sum);
+        return q ? -p[0] * r : p[0] * (us + r);
     }
 };
 
@@ -79,10 +96,12 @@ __device__ __forceinline__ double py_mod360(double a)
 // in the reference's operation order.  Products with 1/2 and 1 are exact, so
 // they ride in the FMA of the sum that follows (one rounding, the sum's), the
 // zero terms fall away (t is finite or NaN), and w2's two halvings become one
-// of the sum: 11 FP64 operations for 27, the same bits.
-__device__ __forceinline__ void bspline_w64(double t, double* w)
+// of the sum: 8 FP64 operations and 3 (integer) products for 27, the same bits.
+template <bool FIT>
+__device__ __forceinline__ void bspline_w64(double t, double* w, unsigned* notes)
 {
-    const double t2 = t * t, t3 = t2 * t, s3 = (1.0 / 6.0) * t3;
+    const double t2 = mul64<FIT>(t, t), t3 = mul64<FIT>(t2, t), s3 = mul64<FIT>(1.0 / 6.0, t3);
+    *notes |= note64(t3);  // the smallest of them (t is below 2)
     w[0] = __fma_rn(-0.5, t, __fma_rn(0.5, t2, -s3)) + 1.0 / 6.0;
     w[1] = __fma_rn(0.5, t3, -t2) + 4.0 / 6.0;
     w[2] = __fma_rn(0.5, (t2 - t3) + t, 1.0 / 6.0);
@@ -99,27 +118,38 @@ __device__ __forceinline__ void bspline_dw64(double t, double* w)
     w[3] = (3.0 / 6.0) * t2 + (0.0 / 6.0) * t + (0.0 / 6.0);
 }
 
-// Cell index and fractional offset along axis d of a coordinate x; dx = x - a.
-// A coordinate beyond the far end b sets *outside (it can only lie in the last
-// cell, so the other cells skip the compare); a NaN coordinate takes any cell
-// (and a NaN offset).  floor() runs beside the FP64 pipe; the cell index comes
-// from the bits of its result, where the conversions to int and back and the
-// two range compares took four FP64-pipe slots an axis.
-__device__ __forceinline__ int spline_locate64(const SplineGrid& g, int d, double x, double dx,
-                                               double* t, bool* outside)
+// One axis of the spline grid (SplineGrid's entries of it)
+struct Axis64 {
+    double a, b, dinv, top;
+    int n;
+};
+
+__device__ __forceinline__ Axis64 axis64(const SplineGrid& g, int d)
 {
-    const double u = dx * g.dinv[d];
+    return {g.a[d], g.b[d], g.dinv[d], g.top[d], g.n[d]};
+}
+
+// Cell index and fractional offset of a coordinate x; dx = x - a.  A coordinate
+// beyond the far end b sets *outside (it can only lie in the last cell, so the
+// other cells skip the compare); a NaN coordinate takes any cell (and a NaN
+// offset).  floor() runs beside the FP64 pipe; the cell index comes from the
+// bits of its result, where the conversions to int and back and the two range
+// compares took four FP64-pipe slots an axis.
+__device__ __forceinline__ int spline_locate64(const Axis64& g, double x, double dx, double* t,
+                                               bool* outside)
+{
+    const double u = dx * g.dinv;
     double fu = floor(u);
-    if (__double_as_longlong(fu) >= __double_as_longlong(g.top[d])) {  // fu >= n - 2 >= 0, or NaN
-        if (x > g.b[d]) *outside = true;
-        fu = g.top[d];
+    if (__double_as_longlong(fu) >= __double_as_longlong(g.top)) {  // fu >= n - 2 >= 0, or NaN
+        if (x > g.b) *outside = true;
+        fu = g.top;
     }
     *t = u - fu;
     const unsigned long long k = (unsigned long long)__double_as_longlong(fu);
     const int sh = 1075 - (int)((k >> 52) & 0x7ff);  // fu = m 2^-sh, m its 53-bit significand
     const unsigned long long m = (k & 0x000fffffffffffffull) | 0x0010000000000000ull;
     const int i = sh > 52 ? 0 : (int)(m >> (sh & 63));
-    return min(max(i, 0), g.n[d] - 2);
+    return min(max(i, 0), g.n - 2);
 }
 
 // x < a by dx = x - a, whose sign is exact: a negative number, not -0, not NaN
@@ -129,128 +159,140 @@ __device__ __forceinline__ bool negative64(double dx)
            0x7ff0000000000000ull;
 }
 
-// One stencil row: w[0] r0 + w[1] r1 + w[2] r2 + w[3] r3 of both components,
-// every product and sum rounded as the reference rounds it.  FIT: the products
-// on the integer pipe (intfp64.h, the same bits).
+__device__ __forceinline__ double pick4(const double* w, int k)
+{
+    return k == 0 ? w[0] : k == 1 ? w[1] : k == 2 ? w[2] : w[3];
+}
+
+// sum_a w0[a] sum_b w1[b] sum_c w2[c] C[it+a, ix+b, iy+c] of one component (c
+// points at it) of the interleaved (u, v) coefficient block, every product and
+// sum rounded as the reference rounds it.
+//
+// FIT: the 84 products on the integer pipe (11 cycles of the SM for 19) beside
+// the FP64 pipe's 63 sums; *notes tells whether all operands were in its range.
+// A time level is one stretch of code without branches, so that the products of
+// one row overlap the sums of another (a range test per row left each warp
+// waiting for one sum after another: 1.5 times the time); the levels are a
+// rolled loop, all sixteen rows at once would outgrow the instruction caches.
 template <bool FIT>
-__device__ __forceinline__ double2 row_dot64(const double* w, double2 r0, double2 r1, double2 r2,
-                                             double2 r3)
+__device__ __forceinline__ double spline_sum64(const double* __restrict__ c, int st, int sx,
+                                               int nt, int it, int ix, int iy, const double* w0,
+                                               const double* w1, const double* w2,
+                                               unsigned* notes)
 {
-    auto mul = [](double a, double b) { return FIT ? ip_mul_fit(a, b) : a * b; };
-    return make_double2(mul(w[0], r0.x) + mul(w[1], r1.x) + mul(w[2], r2.x) + mul(w[3], r3.x),
-                        mul(w[0], r0.y) + mul(w[1], r1.y) + mul(w[2], r2.y) + mul(w[3], r3.y));
-}
-
-// every one of four doubles is in the range of the integer products
-__device__ __forceinline__ bool fit4(double a, double b, double c, double d)
-{
-    return ((((unsigned)__double2hiint(a) - 0x30000000u) |
-             ((unsigned)__double2hiint(b) - 0x30000000u) |
-             ((unsigned)__double2hiint(c) - 0x30000000u) |
-             ((unsigned)__double2hiint(d) - 0x30000000u)) & 0x60000000u) == 0;
-}
-
-// the first term of a sum that starts at 0 (one rounding, the product's), and a
-// further one
-__device__ __forceinline__ double first64(double w, double b)
-{
-    return ip_fits(ip_bits(w), ip_bits(b)) ? ip_mul_fit(w, b) : __fma_rn(w, b, 0.0);
-}
-__device__ __forceinline__ double next64(double s, double w, double b) { return s + ip_mul(w, b); }
-
-// sum_a w0[a] sum_b w1[b] sum_c w2[c] C[it+a, ix+b, iy+c] of the interleaved
-// (u, v) coefficient block.  The 168 products of a point went to the FP64 pipe
-// beside its 126 sums, at 19 cycles of the SM each; on the integer pipe they
-// take 11.  Rows or weights out of the integer arithmetic's range (zeros above
-// all: velocity masked over land, a point on a grid node) take the FP64 pipe.
-// The time levels are a rolled loop: unrolled, the sixteen rows of integer code
-// outgrow the instruction caches.
-__device__ __forceinline__ void spline_sum_uv64(const SplineGrid& g, const double2* __restrict__ c,
-                                                int it, int ix, int iy, const double* w0,
-                                                const double* w1, const double* w2, double* u,
-                                                double* v)
-{
-    const bool wfit = fit4(w2[0], w2[1], w2[2], w2[3]);
-    double au = 0.0, av = 0.0;
+    double au = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) *notes |= note64(w0[k]) | note64(w1[k]) | note64(w2[k]);
 #pragma unroll 1
     for (int a = 0; a < 4; ++a) {
-        double su, sv;
-#pragma unroll
+        double d[4], su;
+        constexpr int kRows = FIT ? 4 : 1;
+#pragma unroll kRows
         for (int b = 0; b < 4; ++b) {
-            const size_t e = (size_t)(it + a) * g.st + (size_t)(ix + b) * g.sx + iy;
-            const double2* row = c + e;
-            double2 r0 = make_double2(0.0, 0.0), r1 = r0, r2 = r0, r3 = r0;
-            if (NBCS_CHECKED(e + 3 < (size_t)g.st * (size_t)(g.n[0] + 2),
-                             NBCS_CHECK_SPLINE_GATHER)) {
-                r0 = __ldg(row);
-                r1 = __ldg(row + 1);
-                r2 = __ldg(row + 2);
-                r3 = __ldg(row + 3);
+            const size_t e = (size_t)(it + a) * st + (size_t)(ix + b) * sx + iy;
+            const double* row = c + 2 * e;
+            double r[4] = {0.0, 0.0, 0.0, 0.0};
+            if (NBCS_CHECKED(e + 3 < (size_t)st * (size_t)(nt + 2), NBCS_CHECK_SPLINE_GATHER)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r[k] = __ldg(row + 2 * k);
             }
-            const bool fit = wfit && fit4(r0.x, r1.x, r2.x, r3.x) && fit4(r0.y, r1.y, r2.y, r3.y);
-            const double2 d = fit ? row_dot64<true>(w2, r0, r1, r2, r3)
-                                  : row_dot64<false>(w2, r0, r1, r2, r3);
-            su = b == 0 ? first64(w1[0], d.x) : next64(su, w1[b], d.x);
-            sv = b == 0 ? first64(w1[0], d.y) : next64(sv, w1[b], d.y);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) *notes |= note64(r[k]);
+            d[b] = mul64<FIT>(w2[0], r[0]) + mul64<FIT>(w2[1], r[1]) + mul64<FIT>(w2[2], r[2]) +
+                   mul64<FIT>(w2[3], r[3]);
+            *notes |= note64(d[b]);
+            const double p = mul64<FIT>(pick4(w1, b), d[b]);
+            su = b ? su + p : FIT ? p : __fma_rn(w1[0], d[0], 0.0);
         }
-        const double wa = a == 0 ? w0[0] : a == 1 ? w0[1] : a == 2 ? w0[2] : w0[3];
-        au = a == 0 ? first64(wa, su) : next64(au, wa, su);
-        av = a == 0 ? first64(wa, sv) : next64(av, wa, sv);
+        *notes |= note64(su);
+        const double wa = pick4(w0, a), p = mul64<FIT>(wa, su);
+        au = a ? au + p : FIT ? p : __fma_rn(wa, su, 0.0);
     }
-    *u = au;
-    *v = av;
+    return au;
 }
 
-// Tricubic evaluation of (u, v) at (t, x, y) with extrapolation mode XM, the
-// extrap_mode of the interpolation package's eval_spline that the reference
-// passes through (flows.py:121):
+// the evaluation on the FP64 pipe: velocity masked over land (coefficients of
+// exactly zero), a point on a grid node (a weight of zero), values beyond the
+// integer arithmetic's range
+static __device__ __noinline__ double spline_plain64(const double* __restrict__ c, int st, int sx,
+                                                     int nt, int it, int ix, int iy, double ft,
+                                                     double fx, double fy)
+{
+    double w0[4], w1[4], w2[4];
+    unsigned notes = 0;
+    bspline_w64<false>(ft, w0, &notes);
+    bspline_w64<false>(fx, w1, &notes);
+    bspline_w64<false>(fy, w2, &notes);
+    return spline_sum64<false>(c, st, sx, nt, it, ix, iy, w0, w1, w2, &notes);
+}
+
+// Tricubic evaluation at (t, x, y) with extrapolation mode XM, the extrap_mode
+// of the interpolation package's eval_spline that the reference passes through
+// (flows.py:121):
 //   0 "constant": 0 strictly outside the grid box;
 //   1 "nearest":  each coordinate clamped into its axis' [a, b];
 //   2 "linear":   the value at the clamped point plus, for each clamped axis
 //                 (t, x, y in that order), the derivative along that axis at
 //                 the clamped point times the distance beyond the box.
+// Lane q of the particle gives its coordinate v of x, y and gets its component:
+// it finds the cell and the weights of its own axis and takes the other axis'
+// from the other lane.
 template <int XM>
-__device__ __forceinline__ void spline_eval_uv64(const SplineGrid& g, const double2* __restrict__ c,
-                                                 double t, double x, double y, double* u,
-                                                 double* v)
+__device__ __forceinline__ double spline_eval64(const SplineGrid& g, const double2* __restrict__ c,
+                                                double t, double v, int q)
 {
-    const double vv[3] = {t, x, y};
-    double dl[3], f[3], w[3][4];
-    int i[3];
-    bool out = false;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        double cl = vv[d];
-        if (XM != 0) cl = vv[d] < g.a[d] ? g.a[d] : (vv[d] > g.b[d] ? g.b[d] : vv[d]);
-        const double dx = cl - g.a[d];
-        if (XM != 0) dl[d] = vv[d] - cl;
-        else if (negative64(dx)) out = true;
-        i[d] = spline_locate64(g, d, cl, dx, &f[d], &out);
+    const Axis64 at = axis64(g, 0);
+    const Axis64 ao = {q ? g.a[2] : g.a[1], q ? g.b[2] : g.b[1], q ? g.dinv[2] : g.dinv[1],
+                       q ? g.top[2] : g.top[1], q ? g.n[2] : g.n[1]};
+    const double* comp = reinterpret_cast<const double*>(c) + q;
+    double ct = t, co = v;
+    if (XM != 0) {
+        ct = t < at.a ? at.a : (t > at.b ? at.b : t);
+        co = v < ao.a ? ao.a : (v > ao.b ? ao.b : v);
     }
-    if (XM == 0 && out) {
-        *u = 0.0;
-        *v = 0.0;
-        return;
-    }
+    const double dt = ct - at.a, dv = co - ao.a;
+    bool out = XM == 0 && (negative64(dt) || negative64(dv));
+    double ft, fo;
+    const int it = spline_locate64(at, ct, dt, &ft, &out);
+    const int io = spline_locate64(ao, co, dv, &fo, &out);
+    const unsigned pm = pair_mask64();
+    if (XM == 0 && __any_sync(pm, out)) return 0.0;
+    const int ip = __shfl_xor_sync(pm, io, 1);
+    const int ix = q ? ip : io, iy = q ? io : ip;
+    double w0[4], wo[4], wx[4], wy[4];
+    unsigned notes = 0;
+    bspline_w64<true>(ft, w0, &notes);
+    bspline_w64<true>(fo, wo, &notes);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) bspline_w64(f[d], w[d]);
-    double au, av;
-    spline_sum_uv64(g, c, i[0], i[1], i[2], w[0], w[1], w[2], &au, &av);
+    for (int k = 0; k < 4; ++k) {
+        const double wp = other64(wo[k]);
+        wx[k] = q ? wp : wo[k];
+        wy[k] = q ? wo[k] : wp;
+    }
+    const double fp = other64(fo), fx = q ? fp : fo, fy = q ? fo : fp;
+    double au = spline_sum64<true>(comp, g.st, g.sx, g.n[0], it, ix, iy, w0, wx, wy, &notes);
+    if (!fits64(notes))
+        au = spline_plain64(comp, g.st, g.sx, g.n[0], it, ix, iy, ft, fx, fy);
     if (XM == 2) {
+        const double dlo = v - co, dlp = other64(dlo);
+        const double f[3] = {ft, fx, fy};
+        const double dl[3] = {t - ct, q ? dlp : dlo, q ? dlo : dlp};
 #pragma unroll 1
         for (int d = 0; d < 3; ++d) {
             if (dl[d] == 0.0 || isnan(dl[d])) continue;
-            double dw[4], gu, gv;
+            double dw[4], p0[4], p1[4], p2[4];
             bspline_dw64(f[d], dw);
-            spline_sum_uv64(g, c, i[0], i[1], i[2], d == 0 ? dw : w[0], d == 1 ? dw : w[1],
-                            d == 2 ? dw : w[2], &gu, &gv);
+            bspline_w64<false>(ft, p0, &notes);
+            bspline_w64<false>(fx, p1, &notes);
+            bspline_w64<false>(fy, p2, &notes);
+            const double gu = spline_sum64<false>(comp, g.st, g.sx, g.n[0], it, ix, iy,
+                                                  d == 0 ? dw : p0, d == 1 ? dw : p1,
+                                                  d == 2 ? dw : p2, &notes);
             const double s = dl[d] * g.dinv[d];
             au = au + s * gu;
-            av = av + s * gv;
         }
     }
-    *u = au;
-    *v = av;
+    return au;
 }
 
 // XM: extrapolation mode (0 constant, 1 nearest, 2 linear)
@@ -260,23 +302,18 @@ struct FlowSpline64 {
     const double2* __restrict__ c;
     double r;
 
-    __device__ __forceinline__ void operator()(double t, const double* y, double* dy,
-                                               const Params& P) const
+    __device__ __forceinline__ double operator()(double t, double y, int q, const Params& P) const
     {
         const double* p = P.v;
-        double tt = p[0] * t;
-        double u, v;
-        if (SPH == 1 || SPH == 2) {
-            double xx = SPH == 1 ? py_mod360(y[0] - 180.0) - 180.0 : py_mod360(y[0]);
-            double yy = y[1];
-            spline_eval_uv64<XM>(g, c, tt, xx, yy, &u, &v);
-            dy[0] = p[0] * u * 180.0 / (NBCS_PI * r * nbcs_cos_deg(yy));
-            dy[1] = p[0] * v * 180.0 / (NBCS_PI * r);
-        } else {
-            spline_eval_uv64<XM>(g, c, tt, y[0], y[1], &u, &v);
-            dy[0] = p[0] * u;
-            dy[1] = p[0] * v;
-        }
+        const double tt = p[0] * t;
+        if (SPH == 0) return p[0] * spline_eval64<XM>(g, c, tt, y, q);
+        // lane 0 holds the longitude, lane 1 the latitude
+        const double lon = SPH == 1 ? py_mod360(y - 180.0) - 180.0 : py_mod360(y);
+        const double w = spline_eval64<XM>(g, c, tt, q ? y : lon, q);
+        // u 180 / (pi r cos(lat)) on lane 0, v 180 / (pi r) on lane 1
+        const double yo = other64(y), pr = NBCS_PI * r;
+        const double den = q ? pr : pr * nbcs_cos_deg(q ? y : yo);
+        return ip_div(p[0] * w * 180.0, ip_reciprocal(den));
     }
 };
 

@@ -19,6 +19,8 @@ void t_mul(const double* a, const double* b, long n, double* o) { for (long i = 
 void t_div(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_div(a[i], ip_reciprocal(b[i])); }
 void t_sqrt(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_sqrt(a[i]); }
 void t_log(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_log(a[i]); }
+void t_sin(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) { double c; ip_sincos(a[i], o + i, &c); if (ip_bits(o[i]) != ip_bits(ip_sin(a[i]))) o[i] = 99.0; } }
+void t_cos(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) { double s; ip_sincos(a[i], &s, o + i); } }
 void t_rsqrt(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_apply_fit(b[i], ip_rsqrt_fit(a[i])); }
 }
 """
@@ -112,3 +114,26 @@ def test_logarithm_and_reciprocal_root(lib):
     b = _numbers(rng, 200000, -200, 200)
     want = b.astype(np.longdouble) / np.sqrt(a.astype(np.longdouble))
     assert _ulps(_call(lib, "t_rsqrt", a, b), want).max() < 0.55
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).nmant < 63, reason="needs an 80-bit long double")
+def test_sine_and_cosine(lib):
+    rng = np.random.default_rng(7)
+    x = np.concatenate([rng.uniform(-64, 64, 200000), rng.uniform(-2, 2, 100000),
+                        np.exp(rng.uniform(-60, 4, 100000)),
+                        np.arange(-80, 81) * (np.pi / 4), np.arange(-40, 41) * (np.pi / 2) * (1 + 1e-12),
+                        [0.0, -0.0, 2.0 ** -27, -(2.0 ** -27), np.nextafter(64.0, 0), 64.0, -100.0,
+                         1e300]])
+    for name, fn in (("t_sin", np.sin), ("t_cos", np.cos)):
+        got, want = _call(lib, name, x, x), fn(x.astype(np.longdouble))
+        # a rounding (0.5 ulp and the series' 2^-60) plus the reduction's 2^-58
+        # absolute; below 2^-27 the argument itself (half an ulp off), and the
+        # library beyond 64 (within an ulp)
+        ulp = np.ldexp(1.0, np.frexp(want.astype(np.float64))[1] - 53)
+        err = np.abs(got.astype(np.longdouble) - want)
+        slack = np.where(np.abs(x) < 0.75, 0.0, 2.0 ** -58)
+        assert np.all(err <= np.where(np.abs(x) < 64, 0.52, 1.0) * ulp + slack), name
+    assert np.all(np.isnan(_call(lib, "t_sin", np.array([np.inf, np.nan]), np.zeros(2))) |
+                  (_call(lib, "t_sin", np.array([np.inf, np.nan]), np.zeros(2)) == 99.0))
+    z = _call(lib, "t_sin", np.array([0.0, -0.0]), np.zeros(2))
+    assert np.array_equal(np.signbit(z), [False, True]) and not z.any()
