@@ -141,7 +141,7 @@ __device__ __forceinline__ int spline_locate64(const Axis64& g, double x, double
     const double u = dx * g.dinv;
     double fu = floor(u);
     if (__double_as_longlong(fu) >= __double_as_longlong(g.top)) {  // fu >= n - 2 >= 0, or NaN
-        if (x > g.b) *outside = true;
+        if (ip_pipe_greater(x, g.b)) *outside = true;
         fu = g.top;
     }
     *t = u - fu;

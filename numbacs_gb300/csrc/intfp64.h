@@ -115,6 +115,23 @@ NBCS_IHD uint32_t ip_estimate(uint32_t fb, bool root)
     return ((yb & 0x7fffffu) | 0x800000u) << 7;
 }
 
+/* The FP64 pipe's operations where they are the exception (operands out of
+ * range, a coordinate in the last cell).  Out of line: in line the compiler
+ * issues them under a false predicate beside the usual path, at the FP64 pipe's
+ * full price. */
+#ifdef __CUDACC__
+static __device__ __noinline__ double ip_pipe_mul(double a, double b) { return a * b; }
+static __device__ __noinline__ double ip_pipe_sub(double a, double b) { return a - b; }
+static __device__ __noinline__ bool ip_pipe_greater(double a, double b) { return a > b; }
+#endif
+#ifdef __CUDA_ARCH__
+#define IP_PIPE_MUL(a, b) ip_pipe_mul(a, b)
+#define IP_PIPE_SUB(a, b) ip_pipe_sub(a, b)
+#else
+#define IP_PIPE_MUL(a, b) ((a) * (b))
+#define IP_PIPE_SUB(a, b) ((a) - (b))
+#endif
+
 #define IP_IMPLICIT 0x0010000000000000ull
 #define IP_FRACTION 0x000fffffffffffffull
 #define IP_SIGN 0x8000000000000000ull
@@ -215,7 +232,7 @@ NBCS_IHD double ip_sqr_or_zero(double a)
 /* a * b */
 NBCS_IHD double ip_mul(double a, double b)
 {
-    return ip_fits(ip_bits(a), ip_bits(b)) ? ip_mul_fit(a, b) : a * b;
+    return ip_fits(ip_bits(a), ip_bits(b)) ? ip_mul_fit(a, b) : IP_PIPE_MUL(a, b);
 }
 
 /* a 2^k, exact */
@@ -223,7 +240,32 @@ NBCS_IHD double ip_scale(double a, int k)
 {
     const ip_u64 u = ip_bits(a);
     return ip_fits(u) ? ip_double(u + ((ip_u64)(int64_t)k << 52))
-                      : a * ip_double((ip_u64)(1023 + k) << 52);
+                      : IP_PIPE_MUL(a, ip_double((ip_u64)(1023 + k) << 52));
+}
+
+/* a - b.  Of the same sign and of exponents at most one apart, as neighbouring
+ * values of a smooth field mostly are, the significands' difference is an
+ * integer of 54 bits at most: exact or half an ulp to round. */
+NBCS_IHD double ip_sub(double a, double b)
+{
+    const ip_u64 ua = ip_bits(a), ub = ip_bits(b);
+    const uint32_t ah = (uint32_t)(ua >> 32), bh = (uint32_t)(ub >> 32);
+    /* exponents (with the sign) one apart or equal: 0, 1 or 2 */
+    const uint32_t da = (ah >> 20) - (bh >> 20) + 1u;
+    if (da > 2u || (int32_t)(ah ^ bh) < 0 || !ip_fits(ua, ub)) return IP_PIPE_SUB(a, b);
+    const ip_u64 A = (((ua & IP_FRACTION) | IP_IMPLICIT)) << (da >> 1);
+    const ip_u64 B = (((ub & IP_FRACTION) | IP_IMPLICIT)) << (da == 0 ? 1 : 0);
+    const int64_t d = (int64_t)(A - B);
+    ip_u64 m = (ip_u64)(d < 0 ? -d : d);
+    if (!m) return 0.0;
+    int e = (int)(((da == 2u ? bh : ah) >> 20) & 0x7ffu);
+    int n = ip_clz64(m) - 11;
+    if (n < 0) {
+        m = (m >> 1) + (m & (m >> 1) & 1u);
+        e += 1;
+        n = 0;
+    }
+    return ip_pack(ua ^ (ip_u64)d, m << n, e - n);
 }
 
 /* A divisor: r = 2^127 / B with the significand B (top bit at 63), to within

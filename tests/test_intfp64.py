@@ -17,6 +17,7 @@ SRC = r"""
 extern "C" {
 void t_mul(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_mul(a[i], b[i]); }
 void t_div(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_div(a[i], ip_reciprocal(b[i])); }
+void t_sub(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_sub(a[i], b[i]); }
 void t_sqrt(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_sqrt(a[i]); }
 void t_log(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_log(a[i]); }
 void t_sin(const double* a, const double*, long n, double* o) { for (long i = 0; i < n; ++i) { double c; ip_sincos(a[i], o + i, &c); if (ip_bits(o[i]) != ip_bits(ip_sin(a[i]))) o[i] = 99.0; } }
@@ -88,6 +89,14 @@ def test_products_quotients_roots_bit_for_bit(lib, span):
             nan = np.isnan(want)
             assert np.array_equal(np.isnan(got), nan), name
             assert np.array_equal(_bits(got)[~nan], _bits(want)[~nan]), name
+        # differences of neighbours: the same exponent, the next one, the next double
+        near = ((a.view(np.uint64) & ~np.uint64((1 << 52) - 1)) |
+                (b.view(np.uint64) & np.uint64((1 << 52) - 1))).view(np.float64)
+        for c in (b, near, near * 2.0, near * 0.5, a, np.nextafter(a, b), -near):
+            want, got = a - c, _call(lib, "t_sub", a, c)
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan)
+            assert np.array_equal(_bits(got)[~nan], _bits(want)[~nan])
         for x in (a, a * a, np.nextafter(a * a, np.inf)):
             want, got = np.sqrt(x), _call(lib, "t_sqrt", x, x)
             nan = np.isnan(want)
