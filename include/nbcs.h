@@ -320,6 +320,21 @@ int nbcs_ridge_pts(const double* f, const double* evec_max, const double* x, int
                    uint8_t* mask_out, double* rpts_full, double* pts_out, int64_t* n_out,
                    void* scratch, size_t scratch_bytes, void* stream);
 
+/* nbcs_ridge_pts plus what ftle_ridges needs (ridges.py:186-229): pt_index
+ * (nx*ny int32) receives the points' linear grid indices, and -- for up to
+ * NBCS_RIDGE_COMPONENTS_MAX points -- comp_pts (2 * NBCS_RIDGE_COMPONENTS_MAX
+ * doubles) the points ordered by their 8-connected component (numbered by first
+ * point in row-major order) and by row-major order inside each, head[0] the
+ * number of points, head[1] that of components and head[2 ..] their sizes
+ * (NBCS_RIDGE_COMPONENTS_MAX + 2 int32).  With more points head[1] is -1 and
+ * comp_pts is left alone. */
+#define NBCS_RIDGE_COMPONENTS_MAX 8192
+int nbcs_ridge_components(const double* f, const double* evec_max, const double* x, int32_t nx,
+                          const double* y, int32_t ny, double sdd_thresh, double percentile,
+                          uint8_t* mask_out, double* pts_out, int32_t* pt_index, int64_t* n_out,
+                          double* comp_pts, int32_t* head, void* scratch, size_t scratch_bytes,
+                          void* stream);
+
 /* nbcs_ridge_pts with the threshold f_min and the grid spacing dx, dy given
  * instead of a percentile of f and x[1] - x[0], y[1] - y[0] (no reference
  * counterpart: a row block of a field sharded over several GPUs takes the

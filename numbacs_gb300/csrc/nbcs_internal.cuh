@@ -107,6 +107,37 @@ inline SplineGrid make_grid(const double* g)
     return s;
 }
 
+// Quotient of an index below 2^31 by a divisor fixed at launch: one high
+// product and a shift (Granlund & Montgomery 1994; with s = ceil(log2 d) and
+// m = ceil(2^(31+s) / d) the error m d - 2^(31+s) is below 2^s, so it is exact
+// for every dividend below 2^31).  A 64-bit division took the better part of a
+// hundred instructions a point.
+struct FastDiv {
+    unsigned m, s, d;
+};
+
+inline FastDiv fast_div(int d)
+{
+    FastDiv f;
+    f.d = (unsigned)d;
+    f.s = 0;
+    while ((1ull << f.s) < (unsigned long long)d) ++f.s;
+    f.m = (unsigned)(((1ull << (31 + f.s)) + (unsigned)d - 1) / (unsigned)d);
+    return f;
+}
+
+__device__ __forceinline__ unsigned div_by(unsigned k, const FastDiv& f)
+{
+    return (unsigned)(((unsigned long long)k * f.m) >> (31 + f.s));
+}
+
+// row i and column j of point k of an (nx, ny) grid
+__device__ __forceinline__ void row_col(long k, const FastDiv& f, int* i, int* j)
+{
+    *i = k < 0x80000000L ? (int)div_by((unsigned)k, f) : (int)(k / (long)f.d);
+    *j = (int)(k - (long)*i * (long)f.d);
+}
+
 int validate_flow(const nbcs_flow* flow, const double* params, int32_t np, int precision);
 
 }  // namespace nbcs

@@ -12,9 +12,7 @@ from .. import _device as D
 from .. import _lib
 
 
-def _run(f, eigvec_max, x, y, sdd_thresh, percentile, want_mask, want_full, f_min=None,
-         dxdy=None):
-    D.require_cuda()
+def _inputs(f, eigvec_max, x, y):
     fd = D.to_dev(f)
     ev = D.to_dev(eigvec_max)
     xd, yd = D.to_dev(x), D.to_dev(y)
@@ -23,6 +21,14 @@ def _run(f, eigvec_max, x, y, sdd_thresh, percentile, want_mask, want_full, f_mi
     nx, ny = fd.shape
     if tuple(ev.shape) != (nx, ny, 2):
         raise ValueError("eigvec_max must have shape (nx, ny, 2)")
+    return fd, ev, xd, yd
+
+
+def _run(f, eigvec_max, x, y, sdd_thresh, percentile, want_mask, want_full, f_min=None,
+         dxdy=None):
+    D.require_cuda()
+    fd, ev, xd, yd = _inputs(f, eigvec_max, x, y)
+    nx, ny = fd.shape
     L = _lib.load()
     nbytes = L.nbcs_ridge_scratch_bytes(nx, ny)
     scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=fd.device)
@@ -109,19 +115,46 @@ def ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, min_ridge_pts
     components ordered by their first grid point in row-major order and
     points within a ridge in row-major order (ridges.py:186-229).
 
-    Mask, ridge points and component labels are computed on the GPU
-    (csrc/ridges.cu, csrc/label.cu); the per-ridge split of the labelled
-    points is a stable sort by label of the (few) ridge pixels.
+    Ridge points, components and their order are computed on the GPU in two
+    launches (csrc/ridges.cu) for up to 8192 ridge points; beyond, the mask is
+    labelled (csrc/label.cu) and the points sorted by label.
     """
+    D.require_cuda()
     as_torch = D.is_torch(f, eigvec_max)
-    _, _, mask, full = _run(f, eigvec_max, x, y, sdd_thresh, percentile, True, True)
-    labels, n = label8(mask)
-    lab = labels.view(-1)
-    idx = torch.nonzero(lab, as_tuple=True)[0]  # ascending: row-major
-    labs = lab.index_select(0, idx).long()
-    order = torch.sort(labs, stable=True).indices
-    pts = full.index_select(0, idx.index_select(0, order))
-    counts = torch.bincount(labs, minlength=n + 1)[1:].tolist()
+    fd, ev, xd, yd = _inputs(f, eigvec_max, x, y)
+    nx, ny = fd.shape
+    if nx * ny > 0x7fffffff:
+        raise ValueError("grids of more than 2^31 - 1 points are not supported")
+    L = _lib.load()
+    nbytes = L.nbcs_ridge_scratch_bytes(nx, ny)
+    scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=fd.device)
+    mask = D.empty((nx, ny), torch.uint8)
+    pts = D.empty((nx * ny, 2))
+    index = D.empty((nx * ny,), torch.int32)
+    n_out = D.empty((1,), torch.int64)
+    cap = _lib.RIDGE_COMPONENTS_MAX
+    comp = D.empty((cap, 2))
+    head = D.empty((cap + 2,), torch.int32)
+    _lib.check(L.nbcs_ridge_components(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
+                                       float(sdd_thresh), float(percentile), D.ptr(mask),
+                                       D.ptr(pts), D.ptr(index), D.ptr(n_out), D.ptr(comp),
+                                       D.ptr(head), D.ptr(scratch), nbytes, D.stream_ptr()))
+    first = head[:1024].tolist()
+    n, ncomp = first[0], first[1]
+    if n < 0:
+        raise RuntimeError("ftle_ridges: the launch did not finish")
+    if ncomp >= 0:
+        counts = first[2:2 + ncomp]
+        if ncomp > len(counts):
+            counts += head[1024:2 + ncomp].tolist()
+        pts = comp[:n].clone()  # the views below do not hold on to the whole buffer
+    else:
+        n = int(n_out.item())
+        labels, ncomp = label8(mask)
+        labs = labels.view(-1).index_select(0, index[:n].long()).long()
+        order = torch.sort(labs, stable=True).indices
+        pts = pts.index_select(0, order)
+        counts = torch.bincount(labs, minlength=ncomp + 1)[1:].tolist()
     ridges, start = [], 0
     for c in counts:
         if c >= min_ridge_pts:
