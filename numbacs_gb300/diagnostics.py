@@ -52,16 +52,28 @@ def ftle_from_eig(eigval_max, T):
     """log(eigval_max) / (2|T|) where eigval_max > 1, else 0."""
     D.require_cuda()
     as_torch = D.is_torch(eigval_max)
-    if isinstance(eigval_max, torch.Tensor) and eigval_max.is_cuda and eigval_max.dtype == torch.float64:
-        e = eigval_max
-        if not e.is_contiguous():
-            e = e.contiguous()
-    else:
-        e = D.to_dev(eigval_max)
-    out = D.empty(tuple(e.shape))
-    _lib.check(_lib.load().nbcs_ftle_from_eig(D.ptr(e), e.numel(), 1, float(T), D.ptr(out),
+    e, stride = eigval_max, 0
+    if isinstance(e, torch.Tensor) and e.is_cuda and e.dtype == torch.float64:
+        stride = _step(e)
+    if stride == 0:
+        e, stride = D.to_dev(e), 1
+    out = D.empty(e.shape)
+    _lib.check(_lib.load().nbcs_ftle_from_eig(D.ptr(e), e.numel(), stride, float(T), D.ptr(out),
                                               D.stream_ptr()))
     return D.finish(out, as_torch)
+
+
+def _step(t):
+    """Distance between the elements of t in C order where it is one and the
+    same (eigvals[..., 1]: 2, read in place; its copy took 15 us of a 1351 x 501
+    field's call), else 0."""
+    if t.is_contiguous():
+        return 1
+    stride = t.stride()
+    for s, ahead, n in zip(stride, stride[1:], t.shape[1:]):
+        if s != ahead * n:
+            return 0
+    return stride[-1]
 
 
 def ftle_evec_2D(flowmap, T, dx, dy, mask=None):

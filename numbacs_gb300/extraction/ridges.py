@@ -24,18 +24,19 @@ def _inputs(f, eigvec_max, x, y):
     return fd, ev, xd, yd
 
 
-def _run(f, eigvec_max, x, y, sdd_thresh, percentile, want_mask, want_full, f_min=None,
-         dxdy=None):
+def _run(f, eigvec_max, x, y, sdd_thresh, percentile, f_min=None, dxdy=None, full_mask=False):
+    """Ridge points (k, 2), or with full_mask (points or zeros (nx*ny, 2), mask
+    (nx, ny)), which are not waited for."""
     D.require_cuda()
     fd, ev, xd, yd = _inputs(f, eigvec_max, x, y)
     nx, ny = fd.shape
     L = _lib.load()
     nbytes = L.nbcs_ridge_scratch_bytes(nx, ny)
     scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=fd.device)
-    mask = D.empty((nx, ny), torch.uint8) if want_mask else None
-    full = D.empty((nx * ny, 2)) if want_full else None
+    mask = D.empty((nx, ny), torch.uint8) if full_mask else None
+    full = D.empty((nx * ny, 2)) if full_mask else None
     pts = D.empty((nx * ny, 2))
-    n_out = D.empty((1,), torch.int64)
+    n_out = D.empty((1,), torch.int64) if full_mask else D.readback((1,), torch.int64)
     if f_min is None:
         _lib.check(L.nbcs_ridge_pts(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
                                     float(sdd_thresh), float(percentile), D.ptr(mask),
@@ -47,7 +48,13 @@ def _run(f, eigvec_max, x, y, sdd_thresh, percentile, want_mask, want_full, f_mi
                                          float(f_min), D.ptr(mask),
                                          D.ptr(full), D.ptr(pts), D.ptr(n_out), D.ptr(scratch),
                                          nbytes, D.stream_ptr()))
-    return pts, n_out, mask, full
+    if full_mask:
+        return full, mask
+    D.synchronize()
+    k = int(n_out)
+    if k < 0:
+        raise RuntimeError("ridge points: the launch did not finish")
+    return pts[:k]
 
 
 def ridge_pts_fmin(f, eigvec_max, x, y, dx, dy, sdd_thresh, f_min):
@@ -55,9 +62,8 @@ def ridge_pts_fmin(f, eigvec_max, x, y, dx, dy, sdd_thresh, f_min):
     row block of a field sharded over several GPUs: the global threshold and
     spacing) -> ridge points (k, 2), row-major."""
     as_torch = D.is_torch(f, eigvec_max)
-    pts, n_out, _, _ = _run(f, eigvec_max, x, y, sdd_thresh, 0, False, False, f_min=f_min,
-                            dxdy=(dx, dy))
-    return D.finish(pts[:int(n_out.item())], as_torch)
+    pts = _run(f, eigvec_max, x, y, sdd_thresh, 0, f_min=f_min, dxdy=(dx, dy))
+    return D.finish(pts, as_torch)
 
 
 def percentile(f, q):
@@ -67,24 +73,23 @@ def percentile(f, q):
     L = _lib.load()
     nbytes = L.nbcs_percentile_scratch_bytes(fd.numel())
     scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=fd.device)
-    out = D.empty((1,))
+    out = D.readback((1,), torch.float64)
     _lib.check(L.nbcs_percentile(D.ptr(fd), fd.numel(), float(q), D.ptr(out), D.ptr(scratch),
                                  nbytes, D.stream_ptr()))
-    return float(out.item())
+    D.synchronize()
+    return float(out)
 
 
 def ftle_ridge_pts(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
     """Sub-pixel ridge points (k, 2), in row-major grid order."""
     as_torch = D.is_torch(f, eigvec_max)
-    pts, n_out, _, _ = _run(f, eigvec_max, x, y, sdd_thresh, percentile, False, False)
-    k = int(n_out.item())
-    return D.finish(pts[:k], as_torch)
+    return D.finish(_run(f, eigvec_max, x, y, sdd_thresh, percentile), as_torch)
 
 
 def _ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
     """(r_pts (nx*ny, 2) zero off the ridge, ridge_bool (nx, ny), nx, ny)."""
     as_torch = D.is_torch(f, eigvec_max)
-    _, _, mask, full = _run(f, eigvec_max, x, y, sdd_thresh, percentile, True, True)
+    full, mask = _run(f, eigvec_max, x, y, sdd_thresh, percentile, full_mask=True)
     nx, ny = mask.shape
     return D.finish(full, as_torch), D.finish(mask.to(torch.bool), as_torch), nx, ny
 
@@ -134,20 +139,19 @@ def ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, min_ridge_pts
     n_out = D.empty((1,), torch.int64)
     cap = _lib.RIDGE_COMPONENTS_MAX
     comp = D.empty((cap, 2))
-    head = D.empty((cap + 2,), torch.int32)
+    head = D.readback((cap + 2,), torch.int32)
     _lib.check(L.nbcs_ridge_components(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
                                        float(sdd_thresh), float(percentile), D.ptr(mask),
                                        D.ptr(pts), D.ptr(index), D.ptr(n_out), D.ptr(comp),
                                        D.ptr(head), D.ptr(scratch), nbytes, D.stream_ptr()))
-    first = head[:1024].tolist()
-    n, ncomp = first[0], first[1]
+    D.synchronize()
+    head = head.numpy()
+    n, ncomp = int(head[0]), int(head[1])
     if n < 0:
         raise RuntimeError("ftle_ridges: the launch did not finish")
     if ncomp >= 0:
-        counts = first[2:2 + ncomp]
-        if ncomp > len(counts):
-            counts += head[1024:2 + ncomp].tolist()
-        pts = comp[:n].clone()  # the views below do not hold on to the whole buffer
+        counts = head[2:2 + ncomp].tolist()
+        pts = comp[:n]
     else:
         n = int(n_out.item())
         labels, ncomp = label8(mask)
@@ -155,10 +159,11 @@ def ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, min_ridge_pts
         order = torch.sort(labs, stable=True).indices
         pts = pts.index_select(0, order)
         counts = torch.bincount(labs, minlength=ncomp + 1)[1:].tolist()
+    if not as_torch:
+        pts = pts.cpu().numpy()  # one copy for all ridges
     ridges, start = [], 0
     for c in counts:
         if c >= min_ridge_pts:
-            r = pts[start:start + c]
-            ridges.append(r if as_torch else r.cpu().numpy())
+            ridges.append(pts.narrow(0, start, c) if as_torch else pts[start:start + c].copy())
         start += c
     return ridges

@@ -119,8 +119,8 @@ class GpuOps:
         """(ridge mask (n, ny) bool, r_pts (n * ny, 2)) with the threshold and
         spacing given."""
         from .extraction.ridges import _run
-        _, _, mask, full = _run(f, evec, x, y, sdd_thresh, 0, True, True, f_min=f_min,
-                                dxdy=(dx, dy))
+        full, mask = _run(f, evec, x, y, sdd_thresh, 0, f_min=f_min, dxdy=(dx, dy),
+                          full_mask=True)
         return mask.to(bool), full
 
     def label8(self, mask):
