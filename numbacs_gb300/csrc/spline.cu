@@ -16,8 +16,13 @@
 //    the same bits; a division 15 cycles of the SM for 137), which leaves two
 //    FP64 sums an element.
 //  - Both velocity components go in one launch (twice the lines in flight), the
-//    loads of a line run a chunk ahead of its recurrence, and one-warp blocks
-//    share the lines out evenly.
+//    loads of a line run two chunks ahead of its recurrence (one chunk, some
+//    2500 cycles, still waited for memory a tenth of the time), and one-warp
+//    blocks share the lines out evenly.
+//  - The table of pivots is read with constant addresses only: a steady chunk
+//    has its pivot in registers, and the out-of-line functions get scalars.
+//    With the table's address given away its reads were generic loads, a fifth
+//    of a warp's time (57, 82 and 62 us for the three passes below).
 //  - The inner elements go in chunks of eight without a branch: whether every
 //    operand fitted the integer arithmetic is asked once a chunk, which is
 //    redone element by element if not.  A branch per product had the products
@@ -25,7 +30,7 @@
 //  - Lines along y, whose elements are adjacent in memory, are transposed
 //    through shared memory (a warp reads 32 lines in 256-byte runs).
 // Both components of a 121 x 217 x 101 block, the passes along t, x and y: 376,
-// 585 and 329 us in six launches -> 57, 83 and 63 us in three.  What is left is
+// 585 and 329 us in six launches -> 51, 66 and 60 us in three.  What is left is
 // latency: an element takes a 64-cycle FP64 sum after an integer product of
 // some 80 cycles, and the x pass has five warps an SM.
 #include "intfp64.h"
@@ -67,36 +72,51 @@ static Pivots pivots()
     return p;
 }
 
-__device__ __forceinline__ int pivot_index(int k) { return k < kPivots ? k : kPivots - 1; }
+__device__ __forceinline__ int pivot_index(int k) { return min(max(k, 0), kPivots - 1); }
 
 // Forward elimination of element k of m (6 f on the right-hand side), r the
-// previous element's; back substitution of element k, next the following one
-__device__ __noinline__ double eliminate(const Pivots& P, int k, int m, double f, double c0,
-                                         double cn1, double r)
+// previous element's and w its pivot's reciprocal; back substitution of element
+// k, next the following one.  (Scalars, not the table: the table's address, once
+// given away, makes every read of it a load from generic memory.)
+__device__ __noinline__ double eliminate1(double w, bool first, bool last, double f, double c0,
+                                          double cn1, double r)
 {
     double rhs = 6.0 * f;
-    if (k == 0) rhs -= c0;
-    if (k == m - 1) rhs -= cn1;
-    return k == 0 ? rhs : rhs - P.w[pivot_index(k - 1)] * r;
+    if (first) rhs -= c0;
+    if (last) rhs -= cn1;
+    return first ? rhs : rhs - w * r;
 }
 
-__device__ __noinline__ double substitute(const Pivots& P, int k, int m, double r, double next)
+__device__ __noinline__ double substitute1(double b, ip_u64 B, ip_u64 rec, bool last, double r,
+                                           double next)
 {
-    return ip_div(k == m - 1 ? r : r - next, P.d[pivot_index(k)]);
+    const ip_divisor d = {rec, B, b};
+    return ip_div(last ? r : r - next, d);
+}
+
+__device__ __forceinline__ double eliminate(const Pivots& P, int k, int m, double f, double c0,
+                                            double cn1, double r)
+{
+    return eliminate1(P.w[pivot_index(k - 1)], k == 0, k == m - 1, f, c0, cn1, r);
+}
+
+__device__ __forceinline__ double substitute(const Pivots& P, int k, int m, double r, double next)
+{
+    const ip_divisor& d = P.d[pivot_index(k)];
+    return substitute1(d.b, d.B, d.r, k == m - 1, r, next);
 }
 
 constexpr int kPfWarp = 32;   // lines per block
 constexpr int kPfChunk = 8;   // elements at a time
 
-// x / (pivot with reciprocal r) of an operand that fits, r rounded down: the
-// quotient lies in [q, q + 4) of the computed one
-__device__ __forceinline__ double pivot_div_fit(double x, ip_u64 r, const ip_divisor& d)
+// x / (a pivot in [2, 4), of reciprocal r and significand B) of an operand that
+// fits, r rounded down: the quotient lies in [q, q + 4) of the computed one
+__device__ __forceinline__ double pivot_div_fit(double x, ip_u64 r, ip_u64 B)
 {
     const ip_u64 u = ip_bits(x);
     const ip_u64 A = ip_left(u);
     ip_u64 q = ip_mulhi(A, r);
-    int e = ip_exponent(u) - 1;  // pivots lie in [2, 8): exponent 1 or, for 4, 2
-    e -= (int)(ip_exponent(ip_bits(d.b)) - 1024);
+    int e = ip_exponent(u) - 1;
     const bool small = !(q >> 63);
     if (small) {
         q <<= 1;
@@ -104,13 +124,18 @@ __device__ __forceinline__ double pivot_div_fit(double x, ip_u64 r, const ip_div
     }
     unsigned up = (unsigned)(q >> 10) & 1u;
     if (((unsigned)q & 0x7ffu) - 0x3fcu < 4u)
-        up = ip_mulhi((q & ~0x7ffull) | 0x400ull, d.B) < (small ? A : A >> 1);
+        up = ip_mulhi((q & ~0x7ffull) | 0x400ull, B) < (small ? A : A >> 1);
     return ip_pack(u, (q >> 11) + up, e);
 }
+
+// The pivots of a chunk whose lowest element is k: past the table's end they are
+// one pivot, in registers
+constexpr int kSteady = kPivots + 1;
 
 // kPfChunk inner elements from k on (none of them the first or the last):
 // without branches, so that the products off the recurrence overlap it.  False
 // when an operand did not fit the integer arithmetic (r is unchanged then).
+template <bool STEADY>
 __device__ __forceinline__ bool eliminate_chunk(const Pivots& P, int k, const double* f, double* r,
                                                 double* out)
 {
@@ -120,7 +145,7 @@ __device__ __forceinline__ bool eliminate_chunk(const Pivots& P, int k, const do
     for (int j = 0; j < kPfChunk; ++j) {
         bad |= ip_bits(f[j]) - 0x3000000000000000ull;
         rhs[j] = ip_mul_fit(6.0, f[j]);
-        w[j] = P.w[pivot_index(k + j - 1)];
+        w[j] = P.w[STEADY ? kPivots - 1 : pivot_index(k + j - 1)];
     }
 #pragma unroll
     for (int j = 0; j < kPfChunk; ++j) {
@@ -134,18 +159,23 @@ __device__ __forceinline__ bool eliminate_chunk(const Pivots& P, int k, const do
 }
 
 // the same of the back substitution, from k downwards
+template <bool STEADY>
 __device__ __forceinline__ bool substitute_chunk(const Pivots& P, int k, const double* r,
                                                  double* next, double* out)
 {
-    ip_u64 bad = 0, rec[kPfChunk];
+    ip_u64 bad = 0, rec[kPfChunk], B[kPfChunk];
     double v = *next;
 #pragma unroll
-    for (int j = 0; j < kPfChunk; ++j) rec[j] = P.d[pivot_index(k - j)].r;
+    for (int j = 0; j < kPfChunk; ++j) {
+        const int i = STEADY ? kPivots - 1 : pivot_index(k - j);
+        rec[j] = P.d[i].r;
+        B[j] = P.d[i].B;
+    }
 #pragma unroll
     for (int j = 0; j < kPfChunk; ++j) {
         const double x = r[j] - v;
         bad |= ip_bits(x) - 0x3000000000000000ull;
-        v = pivot_div_fit(x, rec[j], P.d[pivot_index(k - j)]);
+        v = pivot_div_fit(x, rec[j], B[j]);
         out[j] = v;
     }
     if ((unsigned)(bad >> 32) & 0x60000000u) return false;
@@ -163,8 +193,8 @@ prefilter_lines_kernel(PrefilterIO io, int n, LineSet L, const __grid_constant__
                        int pitch)
 {
     extern __shared__ double sh[];
-    const double* f = io.f[blockIdx.y];
-    double* c = io.c[blockIdx.y];
+    const double* __restrict__ f = blockIdx.y ? io.f[1] : io.f[0];
+    double* c = blockIdx.y ? io.c[1] : io.c[0];
     const int m = n - 2, lane = threadIdx.x;
     const long lines = L.n_outer * L.n_inner;
     const long l0 = (long)blockIdx.x * kPfWarp, l = l0 + lane;
@@ -210,17 +240,19 @@ prefilter_lines_kernel(PrefilterIO io, int n, LineSet L, const __grid_constant__
             r = eliminate(P, 0, m, in[fs], c0, cn1, r);
             out[2 * cs] = r;
         }
-        double buf[kPfChunk], ahead[kPfChunk], res[kPfChunk];
-        if (chunks) {
+        double buf[kPfChunk], ahead[kPfChunk], after[kPfChunk], res[kPfChunk];
 #pragma unroll
-            for (int j = 0; j < kPfChunk; ++j) buf[j] = in[(long)(j + 2) * fs];
+        for (int j = 0; j < kPfChunk; ++j) {
+            buf[j] = chunks > 0 ? in[(long)(j + 2) * fs] : 0.0;
+            ahead[j] = chunks > 1 ? in[(long)(kPfChunk + j + 2) * fs] : 0.0;
         }
         for (int k = 1; k < body; k += kPfChunk) {
-            const bool more = k + kPfChunk < body;
+            const bool more = k + 2 * kPfChunk < body;
 #pragma unroll
             for (int j = 0; j < kPfChunk; ++j)
-                ahead[j] = more ? in[(long)(k + kPfChunk + j + 1) * fs] : 0.0;
-            if (!eliminate_chunk(P, k, buf, &r, res)) {
+                after[j] = more ? in[(long)(k + 2 * kPfChunk + j + 1) * fs] : 0.0;
+            if (!(k >= kSteady ? eliminate_chunk<true>(P, k, buf, &r, res)
+                               : eliminate_chunk<false>(P, k, buf, &r, res))) {
 #pragma unroll 1
                 for (int j = 0; j < kPfChunk; ++j) {
                     r = eliminate(P, k + j, m, in[(long)(k + j + 1) * fs], c0, cn1, r);
@@ -231,7 +263,10 @@ prefilter_lines_kernel(PrefilterIO io, int n, LineSet L, const __grid_constant__
                 for (int j = 0; j < kPfChunk; ++j) out[(long)(k + j + 2) * cs] = res[j];
             }
 #pragma unroll
-            for (int j = 0; j < kPfChunk; ++j) buf[j] = ahead[j];
+            for (int j = 0; j < kPfChunk; ++j) {
+                buf[j] = ahead[j];
+                ahead[j] = after[j];
+            }
         }
 #pragma unroll 1
         for (int k = m > 0 ? body : 0; k < m; ++k) {
@@ -245,16 +280,18 @@ prefilter_lines_kernel(PrefilterIO io, int n, LineSet L, const __grid_constant__
             out[(long)(k + 2) * cs] = next;
             if (k == m - 1) last = next;
         }
-        if (chunks) {
 #pragma unroll
-            for (int j = 0; j < kPfChunk; ++j) buf[j] = out[(long)(body - 1 - j + 2) * cs];
+        for (int j = 0; j < kPfChunk; ++j) {
+            buf[j] = chunks > 0 ? out[(long)(body - 1 - j + 2) * cs] : 0.0;
+            ahead[j] = chunks > 1 ? out[(long)(body - 1 - kPfChunk - j + 2) * cs] : 0.0;
         }
         for (int k = body - 1; k >= kPfChunk; k -= kPfChunk) {
-            const bool more = k - kPfChunk >= 1;
+            const bool more = k - 2 * kPfChunk >= 1;
 #pragma unroll
             for (int j = 0; j < kPfChunk; ++j)
-                ahead[j] = more ? out[(long)(k - kPfChunk - j + 2) * cs] : 0.0;
-            if (!substitute_chunk(P, k, buf, &next, res)) {
+                after[j] = more ? out[(long)(k - 2 * kPfChunk - j + 2) * cs] : 0.0;
+            if (!(k - kPfChunk >= kSteady ? substitute_chunk<true>(P, k, buf, &next, res)
+                                          : substitute_chunk<false>(P, k, buf, &next, res))) {
 #pragma unroll 1
                 for (int j = 0; j < kPfChunk; ++j) {
                     next = substitute(P, k - j, m, out[(long)(k - j + 2) * cs], next);
@@ -265,7 +302,10 @@ prefilter_lines_kernel(PrefilterIO io, int n, LineSet L, const __grid_constant__
                 for (int j = 0; j < kPfChunk; ++j) out[(long)(k - j + 2) * cs] = res[j];
             }
 #pragma unroll
-            for (int j = 0; j < kPfChunk; ++j) buf[j] = ahead[j];
+            for (int j = 0; j < kPfChunk; ++j) {
+                buf[j] = ahead[j];
+                ahead[j] = after[j];
+            }
         }
         if (m > 0 && body > 0 && m > 1) {
             next = substitute(P, 0, m, out[2 * cs], next);
