@@ -326,6 +326,38 @@ NBCS_IHD double ip_div(double a, const ip_divisor& d)
     return a / d.b;
 }
 
+/* 2^64 sqrt(M / 2^64), three units off at most, of M in [2^62, 2^64) and the
+ * estimate Y of its reciprocal root */
+NBCS_IHD ip_u64 ip_root64(ip_u64 M, uint32_t Y)
+{
+    const uint32_t S = (uint32_t)(((ip_u64)(uint32_t)(M >> 32) * Y) >> 31);  /* root 2^31 */
+    const int64_t D = (int64_t)(M - (((ip_u64)S * S) << 2));  /* below 2^43 */
+    const ip_u64 r =
+        ((ip_u64)S << 33) + (ip_u64)(((int64_t)(int32_t)(D >> 13) * (int32_t)Y) >> 18);
+    const int32_t D2 = (int32_t)(M - ip_mulhi(r, r));
+    return r + (ip_u64)(((int64_t)D2 * (int32_t)Y) >> 31);
+}
+
+/* 2^63 / sqrt(M / 2^64), below 2^64, a few units of 2^2 off, of the same */
+NBCS_IHD ip_u64 ip_rroot64(ip_u64 M, uint32_t Y)
+{
+    /* y += y (1 - M y^2) / 2 twice; 1 - M y^2 in units of 2^-62 */
+    const int64_t E = (int64_t)(0x4000000000000000ull - ip_mulhi(M, ((ip_u64)Y * Y) << 2));
+    const ip_u64 r =
+        ((ip_u64)Y << 32) + (ip_u64)(((int64_t)(int32_t)(E >> 12) * (int32_t)Y) >> 19);
+    const int32_t E2 = (int32_t)(0x4000000000000000ull - ip_mulhi(M, ip_mulhi(r, r) << 2));
+    ip_u64 q = r + (ip_u64)(((int64_t)E2 * (int32_t)Y) >> 31);  /* 2^62 / root, 2^62 to 2^63 */
+    if (!(q >> 62)) q = 0x4000000000000000ull;  /* a root just below 1 */
+    return q >> 63 ? ~0ull : q << 1;
+}
+
+/* the estimate of the reciprocal root of M / 2^64, M in [2^62, 2^64) */
+NBCS_IHD uint32_t ip_root_estimate(ip_u64 M)
+{
+    const uint32_t s = (uint32_t)(M >> 63) ^ 1u, h = (uint32_t)(M >> 32) << s;
+    return ip_estimate(((126u - s) << 23) | ((h >> 8) & 0x7fffffu), true);
+}
+
 /* sqrt(x) of a positive normal number */
 NBCS_IHD double ip_sqrt_fit(double x)
 {
@@ -336,12 +368,7 @@ NBCS_IHD double ip_sqrt_fit(double x)
     const ip_u64 M = ((u & IP_FRACTION) | IP_IMPLICIT) << (11 - s);
     const uint32_t Y =
         ip_estimate(((126u - s) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu), true);
-    const uint32_t S = (uint32_t)(((ip_u64)(uint32_t)(M >> 32) * Y) >> 31);  /* root 2^31 */
-    const int64_t D = (int64_t)(M - (((ip_u64)S * S) << 2));  /* below 2^43 */
-    const ip_u64 r =
-        ((ip_u64)S << 33) + (ip_u64)(((int64_t)(int32_t)(D >> 13) * (int32_t)Y) >> 18);
-    const int32_t D2 = (int32_t)(M - ip_mulhi(r, r));
-    const ip_u64 q = r + (ip_u64)(((int64_t)D2 * (int32_t)Y) >> 31);  /* three units off at most */
+    const ip_u64 q = ip_root64(M, Y);
     uint32_t up = (uint32_t)(q >> 10) & 1u;
     if (((uint32_t)q & 0x7ffu) - (0x400u - 6u) < 12u) {
         const ip_u64 mid = (q & ~0x7ffull) | 0x400ull;
@@ -372,15 +399,8 @@ NBCS_IHD ip_factor ip_rsqrt_fit(double x)
     const ip_u64 M = ((u & IP_FRACTION) | IP_IMPLICIT) << (11 - s);
     const uint32_t Y =
         ip_estimate(((126u - s) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu), true);
-    /* y += y (1 - M y^2) / 2 twice; 1 - M y^2 in units of 2^-62 */
-    const int64_t E = (int64_t)(0x4000000000000000ull - ip_mulhi(M, ((ip_u64)Y * Y) << 2));
-    const ip_u64 r =
-        ((ip_u64)Y << 32) + (ip_u64)(((int64_t)(int32_t)(E >> 12) * (int32_t)Y) >> 19);
-    const int32_t E2 = (int32_t)(0x4000000000000000ull - ip_mulhi(M, ip_mulhi(r, r) << 2));
-    ip_u64 q = r + (ip_u64)(((int64_t)E2 * (int32_t)Y) >> 31);  /* 2^62 / root, 2^62 to 2^63 */
     ip_factor f;
-    if (!(q >> 62)) q = 0x4000000000000000ull;  /* a root just below 1 */
-    f.r = q >> 63 ? ~0ull : q << 1;
+    f.r = ip_rroot64(M, Y);
     f.e = (1023 * 3 - 1 - e + (int)(1u - s)) >> 1;
     return f;
 }
