@@ -134,7 +134,9 @@ __device__ __forceinline__ void tensor_of(const Diffs& D, const ip_divisor& dx2,
     using A = Arith<FIT>;
     const double dxdx = A::div(D.i.x, dx2), dxdy = A::div(D.j.x, dy2);
     const double dydx = A::div(D.i.y, dx2), dydy = A::div(D.j.y, dy2);
-    *b = A::mul(dxdx, dxdy) + A::mul(dydx, dydy);
+    // b's products on the FP64 pipe even the two pipes out: ftle_kernel 2001 x
+    // 1501 90 -> 86 us, with a's too 92
+    *b = dxdx * dxdy + dydx * dydy;
     *a = A::mul(dxdx, dxdx) + A::mul(dydx, dydx);
     *d = A::mul(dxdy, dxdy) + A::mul(dydy, dydy);
 }
