@@ -16,13 +16,14 @@
 // inverse spacing (n - 1) / (b - a) and three explicit-FMA lerps per component,
 // the same operations as the oracle.
 //
-// What bounds it: the FP64 pipe, 19 cycles of the SM an operation; the stack is
-// read from HBM once (a tenth of the time).  Of the 18 operations a map needs,
-// the two scalings, the two cell offsets and four of the six differences run on
-// the integer pipe (intfp64.h, the same bits), which evens out the two pipes,
-// and the tests of the box, of NaN and the cell's index come from bit patterns:
-// ten more FP64-pipe slots a map before.  72 maps of 676 x 251: 729 -> 349 us
-// (368 us with all six differences on the integer pipe).
+// What bounds it: the FP64 pipe, 19 cycles of the SM an operation, and the
+// integer instructions beside it; the stack is read from HBM once (a tenth of the
+// time).  Of the 18 operations a map needs, the two scalings, the two cell offsets
+// (the low bits of the scaled coordinate) and five of the six differences run on
+// the integer pipe (intfp64.h, the same bits), which evens out the two pipes, and
+// the tests of the box, of NaN and the cell's index come from bit patterns.  72
+// maps of 676 x 251: 729 us with everything on the FP64 pipe, 302 us as it is
+// (305 us with four of the differences on the integer pipe, 329 us with all six).
 #include "intfp64.h"
 #include "nbcs_internal.cuh"
 
@@ -50,16 +51,21 @@ __device__ __forceinline__ int lin_locate(const UAxis& A, double v, double* lam,
     const double d = v - A.a;
     if (ip_bits(d) - 0x8000000000000001ull < 0x7ff0000000000000ull) *out = true;
     const double u = ip_mul(d, A.dinv);
-    double fu = floor(u);
-    if ((long long)ip_bits(fu) >= (long long)ip_bits(A.top)) {  // u >= n - 2, or NaN
-        if (ip_pipe_greater(v, A.b)) *out = true;
-        fu = A.top;
-    }
-    *lam = ip_sub(u, fu);
-    const unsigned long long k = ip_bits(fu);
-    const int sh = 1075 - (int)((k >> 52) & 0x7ff);
-    const int i = sh > 52 ? 0 : (int)(((k & IP_FRACTION) | IP_IMPLICIT) >> (sh & 63));
-    return min(max(i, 0), A.n - 2);
+    const ip_u64 ub = ip_bits(u);
+    // u >= n - 2 (or next below it), or NaN; by the upper halves: the compiler
+    // makes an FP64 compare of the 64-bit one
+    if (__double2hiint(u) >= __double2hiint(A.top) && ip_pipe_greater(v, A.b)) *out = true;
+    // u = M 2^-sh; the cell and what is left of it, exact
+    const int sh = 1075 - ip_exponent(ub);
+    const ip_u64 M = (ub & IP_FRACTION) | IP_IMPLICIT;
+    int i = sh > 52 ? 0 : (int)(M >> (sh & 63));
+    i = min(max(i, 0), A.n - 2);
+    const ip_u64 m = M - ((ip_u64)i << (sh & 63));
+    const int n = ip_clz64(m);
+    *lam = sh > 52 ? ip_double(ub & ~IP_SIGN)
+           : m     ? ip_pack(0, m << (n - 11), 1086 - n - sh)
+                   : 0.0;
+    return i;
 }
 
 __device__ __forceinline__ double2 bilinear2(const double2* __restrict__ f, const UGrid2& g,
@@ -70,7 +76,10 @@ __device__ __forceinline__ double2 bilinear2(const double2* __restrict__ f, cons
     const int i = lin_locate(g.x, px, &l0, &out);
     const int j = lin_locate(g.y, py, &l1, &out);
     if (out) return make_double2(0.0, 0.0);
-    if (nan64(px) || nan64(py)) return make_double2(px + py, px + py);  // NaN in, NaN out
+    if (nan64(px) || nan64(py)) {
+        const double n = ip_pipe_sub(px, ip_neg(py));  // NaN in, NaN out
+        return make_double2(n, n);
+    }
     if (!NBCS_CHECKED(i >= 0 && i <= g.x.n - 2 && j >= 0 && j <= g.y.n - 2,
                       NBCS_CHECK_COMPOSE_GATHER))
         return make_double2(0.0, 0.0);
@@ -83,7 +92,7 @@ __device__ __forceinline__ double2 bilinear2(const double2* __restrict__ f, cons
     const double ay = __fma_rn(l1, ip_sub(f01.y, f00.y), f00.y);
     const double by = __fma_rn(l1, ip_sub(f11.y, f10.y), f10.y);
     v.x = __fma_rn(l0, bx - ax, ax);
-    v.y = __fma_rn(l0, by - ay, ay);
+    v.y = __fma_rn(l0, ip_sub(by, ay), ay);
     return v;
 }
 

@@ -243,29 +243,25 @@ NBCS_IHD double ip_scale(double a, int k)
                       : IP_PIPE_MUL(a, ip_double((ip_u64)(1023 + k) << 52));
 }
 
-/* a - b.  Of the same sign and of exponents at most one apart, as neighbouring
- * values of a smooth field mostly are, the significands' difference is an
- * integer of 54 bits at most: exact or half an ulp to round. */
+/* a - b of operands whose exponents are at most nine apart (of which one fits,
+ * then: both are far from the ends of the exponent range): the significands'
+ * sum or difference is exact in 63 bits, and rounded once */
 NBCS_IHD double ip_sub(double a, double b)
 {
     const ip_u64 ua = ip_bits(a), ub = ip_bits(b);
-    const uint32_t ah = (uint32_t)(ua >> 32), bh = (uint32_t)(ub >> 32);
-    /* exponents (with the sign) one apart or equal: 0, 1 or 2 */
-    const uint32_t da = (ah >> 20) - (bh >> 20) + 1u;
-    if (da > 2u || (int32_t)(ah ^ bh) < 0 || !ip_fits(ua, ub)) return IP_PIPE_SUB(a, b);
-    const ip_u64 A = (((ua & IP_FRACTION) | IP_IMPLICIT)) << (da >> 1);
-    const ip_u64 B = (((ub & IP_FRACTION) | IP_IMPLICIT)) << (da == 0 ? 1 : 0);
-    const int64_t d = (int64_t)(A - B);
-    ip_u64 m = (ip_u64)(d < 0 ? -d : d);
+    const int ea = ip_exponent(ua), eb = ip_exponent(ub), apart = ea - eb;
+    if ((uint32_t)(apart + 9) > 18u || !ip_fits(ua)) return IP_PIPE_SUB(a, b);
+    const int sa = 9 + (apart < 0 ? apart : 0), sb = 9 - (apart > 0 ? apart : 0);
+    const ip_u64 A = ((ua & IP_FRACTION) | IP_IMPLICIT) << sa;
+    const ip_u64 B = ((ub & IP_FRACTION) | IP_IMPLICIT) << sb;
+    const ip_u64 opposite = (ip_u64)((int64_t)(ua ^ ub) >> 63);
+    const int64_t d = (int64_t)(A - ((B ^ opposite) - opposite));
+    const ip_u64 m = (ip_u64)(d < 0 ? -d : d);
     if (!m) return 0.0;
-    int e = (int)(((da == 2u ? bh : ah) >> 20) & 0x7ffu);
-    int n = ip_clz64(m) - 11;
-    if (n < 0) {
-        m = (m >> 1) + (m & (m >> 1) & 1u);
-        e += 1;
-        n = 0;
-    }
-    return ip_pack(ua ^ (ip_u64)d, m << n, e - n);
+    const int n = ip_clz64(m);
+    const ip_u64 L = m << n, q = L >> 11;
+    const uint32_t up = ((uint32_t)L & 0x7ffu) + ((uint32_t)q & 1u) > 0x400u ? 1u : 0u;
+    return ip_pack(ua ^ (ip_u64)d, q + up, ea + 11 - sa - n);
 }
 
 /* A divisor: r = 2^127 / B with the significand B (top bit at 63), to within

@@ -146,3 +146,19 @@ def test_sine_and_cosine(lib):
                   (_call(lib, "t_sin", np.array([np.inf, np.nan]), np.zeros(2)) == 99.0))
     z = _call(lib, "t_sin", np.array([0.0, -0.0]), np.zeros(2))
     assert np.array_equal(np.signbit(z), [False, True]) and not z.any()
+
+
+@pytest.mark.parametrize("apart", range(-11, 12))
+def test_differences_of_every_gap(lib, apart):
+    """exponents up to nine apart and beyond, both signs, low bits that make
+    ties: the same bits as the hardware's"""
+    rng = np.random.default_rng(100 + apart)
+    a = np.ldexp(rng.uniform(1.0, 2.0, 20000), rng.integers(-40, 40, 20000))
+    b = np.ldexp(rng.uniform(1.0, 2.0, 20000), np.frexp(a)[1] - 1 - apart)
+    keep = np.uint64(0xffffffffffffffff) << rng.integers(0, 53, 20000).astype(np.uint64)
+    for x, y in ((a, b), (a, (b.view(np.uint64) & keep).view(np.float64)),
+                 ((a.view(np.uint64) & keep).view(np.float64), b),
+                 (a, (b.view(np.uint64) | ~keep & np.uint64((1 << 52) - 1)).view(np.float64))):
+        for s in (1.0, -1.0):
+            for t in (1.0, -1.0):
+                assert np.array_equal(_bits(_call(lib, "t_sub", s * x, t * y)), _bits(s * x - t * y))
