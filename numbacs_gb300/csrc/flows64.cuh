@@ -58,15 +58,26 @@ struct FlowBickley64 {
         const double Y = ip_div(Yv, ip_reciprocal(p[2]));
         const double ch = cosh(Y), th = tanh(Y);
         const double sech2 = quot64(1.0, ip_mul(ch, ch));
-        // lane 0 takes the cosines, lane 1 the sines
+        // lane 0 needs the cosines, lane 1 the sines; of the first two waves each
+        // lane evaluates its own (the library's functions: the jet is so chaotic
+        // that another last bit leaves 1e-9 of the reference's result within days)
         double tr[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 2; ++k) {
+            const int w = k ? 2 : q;
             double s, c;
-            ip_sincos(ip_mul(p[6 + k], X - ip_mul(p[9 + k], tt)), &s, &c);
-            tr[k] = q ? ip_mul(p[3 + k], p[6 + k]) : p[3 + k];
-            tr[k] = ip_mul(tr[k], q ? s : c);
+            sincos(ip_mul(w == 2 ? p[8] : w ? p[7] : p[6],
+                          X - ip_mul(w == 2 ? p[11] : w ? p[10] : p[9], tt)), &s, &c);
+            if (k == 0) {
+                const double theirs = other64(q ? c : s);
+                tr[0] = q ? theirs : c;
+                tr[1] = q ? s : theirs;
+            } else {
+                tr[2] = q ? s : c;
+            }
         }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) tr[k] = ip_mul(q ? ip_mul(p[3 + k], p[6 + k]) : p[3 + k], tr[k]);
         const double sum = tr[0] + tr[1] + tr[2];
         // dx = U sech^2 + 2 U tanh sech^2 (sum A cos), dy = -(U L sech^2 (sum A k sin))
         const double us = ip_mul(q ? ip_mul(p[1], p[2]) : p[1], sech2);
