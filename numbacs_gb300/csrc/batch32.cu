@@ -99,9 +99,9 @@ batch32_kernel(BatchHeader* hdr, const DevFlow32* __restrict__ flows,
 }
 
 // Tile schedule, one launch per flow class: block b integrates tile b of the
-// class's fields (field table ordered longest first), with the single-field
-// integrator's block (256 threads), tile map (16 x 8 particles at two lanes
-// a particle, 32 x 8 at one) and register budget (3 resident blocks).  The
+// class's fields (field table ordered longest first), 256 threads a block, with
+// the single-field integrator's tile map (16 x 8 particles at two lanes a
+// particle, 32 x 8 at one) and register budget (24 resident warps).  The
 // kernel is instantiated for one right-hand side, so it keeps the
 // single-field kernel's 80 registers where one kernel for every flow kind
 // took 128 (2 blocks per SM); each particle's arithmetic is the single-field
@@ -122,12 +122,12 @@ struct FlowFromDev<FlowSpline32<SPH, LP, EX>> {
 };
 
 template <class Flow, bool UNIFORM>
-__global__ void __launch_bounds__(kFm32Block, kFm32MinBlocks)
+__global__ void __launch_bounds__(kClass32Block, kClass32MinBlocks)
 batch32_class_kernel(Flow fl0, const DevFlow32* __restrict__ flows,
                      const DevField* __restrict__ fields, int nfields, int nmax)
 {
     constexpr int LP = Flow::LP;
-    constexpr int KS = kFm32Block / LP;  // one stage column per particle, shared by its lanes
+    constexpr int KS = kClass32Block / LP;  // one stage column per particle, shared by its lanes
     __shared__ float2 ks[12 * KS];
     __shared__ ParamsF sP;  // the block's field is uniform: its parameters once per block
     float2* kc = ks + threadIdx.x / LP;
@@ -135,10 +135,10 @@ batch32_class_kernel(Flow fl0, const DevFlow32* __restrict__ flows,
     const DevField& F = fields[batch_find<kByTile>(fields, nfields, b)];
     if (threadIdx.x < NBCS_MAX_PARAMS) sP.v[threadIdx.x] = (float)F.P.v[threadIdx.x];
     __syncthreads();
-    const long t = (long)(b - F.tile0) * kFm32Block + threadIdx.x;
+    const long t = (long)(b - F.tile0) * kClass32Block + threadIdx.x;
     int i, j;
     // the lanes of a group share the particle: they leave together
-    if (!tile_particle<LP, kFm32Block, kFm32TileJ>(t, F.nx, F.ny, &i, &j)) return;
+    if (!tile_particle<LP, kClass32Block, kFm32TileJ>(t, F.nx, F.ny, &i, &j)) return;
     const long p = (long)i * F.ny + j;
     double r0 = 0.0, r1 = 0.0;
     int st = NBCS_PARTICLE_MASKED, a = 0, rj = 0, nf = 0;
@@ -161,10 +161,10 @@ static int launch_class(const nbcs_batch_class& c, const Flow& fl, const DevFlow
                         const DevField* fields, int nmax, cudaStream_t s)
 {
     if (c.flow >= 0)
-        batch32_class_kernel<Flow, true><<<(unsigned)c.tiles, kFm32Block, 0, s>>>(
+        batch32_class_kernel<Flow, true><<<(unsigned)c.tiles, kClass32Block, 0, s>>>(
             fl, flows, fields + c.field0, c.nfields, nmax);
     else
-        batch32_class_kernel<Flow, false><<<(unsigned)c.tiles, kFm32Block, 0, s>>>(
+        batch32_class_kernel<Flow, false><<<(unsigned)c.tiles, kClass32Block, 0, s>>>(
             fl, flows, fields + c.field0, c.nfields, nmax);
     NBCS_LAUNCH_CHECK();
     return NBCS_OK;
@@ -372,8 +372,8 @@ extern "C" int nbcs_batch_prepare(const nbcs_flow* flows, int32_t nflows, const 
         chunks += (long long)((F.nx + kBatchTileI - 1) / kBatchTileI) * ((F.ny + tj - 1) / tj);
         if (F.ftle) blocks += (n + kFtleBlock - 1) / kFtleBlock;
         // block tile of the class kernels: (ti x tj) particles
-        const int ti = D.lp == 2 ? TileShape<2, kFm32Block>::TI : TileShape<1, kFm32Block>::TI;
-        const int tjt = D.lp == 2 ? TileShape<2, kFm32Block>::TJ : TileShape<1, kFm32Block>::TJ;
+        const int ti = D.lp == 2 ? TileShape<2, kClass32Block>::TI : TileShape<1, kClass32Block>::TI;
+        const int tjt = D.lp == 2 ? TileShape<2, kClass32Block>::TJ : TileShape<1, kClass32Block>::TJ;
         const long long ft = (long long)((F.nx + ti - 1) / ti) * ((F.ny + tjt - 1) / tjt);
         class_tiles += ft;
         C.tiles += ft;

@@ -84,18 +84,25 @@ struct FlowmapArgs {
     int nyv() const { return aux.n > 0 ? ny * aux.n : ny; }
 };
 
-// Threads per block of the single-field integrator, and the width in y of the
-// particle tile a block integrates: at LP = 2 a block takes a 16 x 8 tile of
-// the grid (8 warps, each a 4 x 4 sub-tile).  Measured on the geophysical
-// spline workload (676 x 251 particles): 128-thread 8 x 8 tiles 5.52 ms,
-// 256-thread 16 x 8 tiles 5.24 ms, 8 x 16 tiles 5.36 ms, 32 x 4 tiles 5.43
-// ms; warps of one block share L1 lines of neighbouring trajectories, and the
-// flow is mostly zonal.  The minimum of 3 resident blocks gives the compiler
-// 85 registers a thread; it takes 80 with no spills (24 warps per SM), 5.08
-// ms; a 64-register cap with 4 blocks spilled and took 5.40 ms.
-constexpr int kFm32Block = 256;
+// Threads per block of the mixed integrators, and the width in y of the particle
+// tile a block integrates: at LP = 2 a block takes an 8 x 8 tile of the grid (4
+// warps, each a 4 x 4 sub-tile).  Warps of one block share L1 lines of
+// neighbouring trajectories; smaller blocks share out a grid of a few blocks per
+// SM more evenly and leave their place sooner when a trajectory lags.  Geophysical
+// flow map (rtol 3e-9) with 256-thread 16 x 8, 128-thread 8 x 8 and 64-thread 8 x 4
+// tiles: 338 x 126 particles 2.92, 2.67 and 2.78 ms, 676 x 251 6.70, 6.65 and
+// (rtol 1e-7) 3.68, 3.68 and 3.96 ms, 1351 x 501 21.4 and 21.3 ms; double gyre
+// 401 x 201 134, 120 and 119 us.  The minimum of 6 resident blocks gives the
+// compiler 85 registers a thread; it takes 80 with no spills (24 warps per SM).
+constexpr int kFm32Block = 128;
 constexpr int kFm32TileJ = 8;
-constexpr int kFm32MinBlocks = 3;
+constexpr int kFm32MinBlocks = 6;
+
+// The same of the batch's class launches, whose many blocks share the SMs evenly
+// anyway: six geophysical fields and a jet 23.1 ms with 256-thread blocks, 24.1
+// with 128.
+constexpr int kClass32Block = 256;
+constexpr int kClass32MinBlocks = 3;
 
 int launch_flowmap64(const nbcs_flow* flow, const FlowmapArgs& a);
 int launch_flowmap32(const nbcs_flow* flow, const FlowmapArgs& a);
