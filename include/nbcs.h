@@ -313,7 +313,9 @@ int nbcs_percentile(const double* f, int64_t n, double q, double* out, void* scr
  * Writes mask_out (nx,ny) u8 if not NULL, rpts_full (nx*ny,2) if not NULL
  * (zeros off the ridge, as _ftle_ridges returns), the row-major compacted
  * points to pts_out (capacity nx*ny rows) and their count to *n_out
- * (device int64).  percentile == 0 means threshold 0 (ridges.py:48-49). */
+ * (int64; like every small result here in device memory or in page-locked
+ * host memory, which can be read after a synchronisation).  percentile == 0
+ * means threshold 0 (ridges.py:48-49). */
 size_t nbcs_ridge_scratch_bytes(int32_t nx, int32_t ny);
 int nbcs_ridge_pts(const double* f, const double* evec_max, const double* x, int32_t nx,
                    const double* y, int32_t ny, double sdd_thresh, double percentile,

@@ -380,40 +380,6 @@ NBCS_IHD double ip_sqrt(double x)
     return ip_fits(u) && !(u >> 63) ? ip_sqrt_fit(x) : sqrt(x);
 }
 
-/* 1 / sqrt(x) of a positive normal number as a significand r (2^63 to 2^64, a
- * few units of 2^-61 off) and the biased exponent e that belongs to it */
-struct ip_factor {
-    ip_u64 r;
-    int e;
-};
-
-NBCS_IHD ip_factor ip_rsqrt_fit(double x)
-{
-    const ip_u64 u = ip_bits(x);
-    const int e = ip_exponent(u);
-    const uint32_t s = (uint32_t)e & 1u;
-    const ip_u64 M = ((u & IP_FRACTION) | IP_IMPLICIT) << (11 - s);
-    const uint32_t Y =
-        ip_estimate(((126u - s) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu), true);
-    ip_factor f;
-    f.r = ip_rroot64(M, Y);
-    f.e = (1023 * 3 - 1 - e + (int)(1u - s)) >> 1;
-    return f;
-}
-
-/* a * f, within 0.51 ulp, of an operand that fits */
-NBCS_IHD double ip_apply_fit(double a, const ip_factor& f)
-{
-    const ip_u64 u = ip_bits(a);
-    ip_u64 q = ip_mulhi(ip_left(u), f.r);
-    int e = ip_exponent(u) + f.e - 1022;
-    if (!(q >> 63)) {
-        q <<= 1;
-        e -= 1;
-    }
-    return ip_pack(u, (q >> 11) + ((q >> 10) & 1), e);
-}
-
 struct ip_log_entry {
     uint32_t c;   /* 2^10 times a reciprocal of 1 + i / 128, rounded up */
     ip_u64 l;     /* -log(c 2^-10) in units of 2^-64 */

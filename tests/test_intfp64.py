@@ -14,6 +14,38 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SRC = r"""
 #include "intfp64.h"
+// b / sqrt(a) by ip_rroot64's significand (2^63 to 2^64)
+struct ip_factor {
+    ip_u64 r;
+    int e;
+};
+
+static inline ip_factor ip_rsqrt_fit(double x)
+{
+    const ip_u64 u = ip_bits(x);
+    const int e = ip_exponent(u);
+    const uint32_t s = (uint32_t)e & 1u;
+    const ip_u64 M = ((u & IP_FRACTION) | IP_IMPLICIT) << (11 - s);
+    const uint32_t Y =
+        ip_estimate(((126u - s) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu), true);
+    ip_factor f;
+    f.r = ip_rroot64(M, Y);
+    f.e = (1023 * 3 - 1 - e + (int)(1u - s)) >> 1;
+    return f;
+}
+
+/* a * f, within 0.51 ulp, of an operand that fits */
+static inline double ip_apply_fit(double a, const ip_factor& f)
+{
+    const ip_u64 u = ip_bits(a);
+    ip_u64 q = ip_mulhi(ip_left(u), f.r);
+    int e = ip_exponent(u) + f.e - 1022;
+    if (!(q >> 63)) {
+        q <<= 1;
+        e -= 1;
+    }
+    return ip_pack(u, (q >> 11) + ((q >> 10) & 1), e);
+}
 extern "C" {
 void t_mul(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_mul(a[i], b[i]); }
 void t_div(const double* a, const double* b, long n, double* o) { for (long i = 0; i < n; ++i) o[i] = ip_div(a[i], ip_reciprocal(b[i])); }
