@@ -81,9 +81,9 @@ struct Arith {
     }
 };
 
-// Differences in [2^-64, 2^64) and a spacing in [2^-32, 2^32): gradients in
-// [2^-97, 2^97), the tensor's entries below 2^196 and, where a sum of theirs
-// cancels without being zero, above 2^-248, their squares in the normal range.
+// Differences in [2^-63, 2^65) and a spacing in [2^-32, 2^31): gradients in
+// [2^-95, 2^96], the tensor's entries below 2^194 and, where a sum of theirs
+// cancels without being zero, above 2^-244, their squares in the normal range.
 __device__ __forceinline__ bool ordinary_diffs(double2 p, double2 q)
 {
     return ((((uint32_t)__double2hiint(p.x) - 0x3c000000u) |
@@ -95,12 +95,6 @@ __device__ __forceinline__ bool ordinary_diffs(double2 p, double2 q)
 static bool ordinary_spacing(double dx, double dy)
 {
     return fabs(dx) >= 0x1p-32 && fabs(dx) < 0x1p31 && fabs(dy) >= 0x1p-32 && fabs(dy) < 0x1p31;
-}
-
-// the same of the reciprocals 1 / (2 dx), 1 / (2 dy) that a field of a batch holds
-__device__ __forceinline__ bool ordinary_recip(double r)
-{
-    return (((uint32_t)__double2hiint(r) - 0x3e000000u) & 0x7fffffffu) < 0x04000000u;
 }
 
 // differences across a point: along x and along y of the flow map (x, y)
@@ -120,7 +114,8 @@ __device__ __forceinline__ Diffs diffs_at(const double2* __restrict__ F, long k,
 }
 
 // the whole warp takes the general form when one of its points needs it: two
-// forms one after the other would cost more than the slower one
+// forms one after the other would cost more than the slower one (only where the
+// two give the same bits: a result must not depend on a point's neighbours)
 __device__ __forceinline__ bool all_ordinary(const Diffs& d, bool spacing)
 {
     return __all_sync(__activemask(), spacing && ordinary_diffs(d.i, d.j));
@@ -327,6 +322,15 @@ ceig_aux_kernel(const double2* __restrict__ F, int nx, FastDiv ny, int eig_main,
     }
 }
 
+// whether the reciprocals 1 / (2 dx), 1 / (2 dy) of the spacing are in [2^-31, 2^33)
+// (gradients of ordinary differences then in [2^-94, 2^98)): the fused entry
+// point and the fields of a batch ask the same of the same numbers
+__host__ __device__ __forceinline__ bool ordinary_recips(double rdx, double rdy)
+{
+    return ((((uint32_t)(ip_bits(rdx) >> 32) - 0x3e000000u) |
+             ((uint32_t)(ip_bits(rdy) >> 32) - 0x3e000000u)) & 0x7c000000u) == 0;
+}
+
 // FTLE and eigvec_max of one point for the fused ftle_evec_2D entry point: the
 // stencil, tensor and larger eigenvalue of ftle_grid_2D / C_eig_2D, with the
 // divisions that only scale -- the central differences' 1 / (2 dx), 1 / (2 dy)
@@ -505,8 +509,11 @@ __device__ __forceinline__ void ftle_evec_point(const double2* __restrict__ F, l
                                                 double* f, double2* v)
 {
     const Diffs D = diffs_at(F, k, ny);
-    const double l1 = all_ordinary(D, spacing) ? eigvec_max_fixed(D, rdx, rdy, &v->x, &v->y)
-                                               : eigvec_max(D, rdx, rdy, &v->x, &v->y);
+    // by the point's own differences (the two forms' last bits differ, and a point
+    // has the same result in any row block and any batch)
+    const double l1 = spacing && ordinary_diffs(D.i, D.j)
+                          ? eigvec_max_fixed(D, rdx, rdy, &v->x, &v->y)
+                          : eigvec_max(D, rdx, rdy, &v->x, &v->y);
     *f = ftle_of(l1, rden);
 }
 
@@ -557,7 +564,7 @@ ftle_batch_kernel(const DevField* __restrict__ fields, int nfields, long long to
         const int j = (int)(k - (long)i * F.ny);
         if (i >= 1 && i < F.nx - 1 && j >= 1 && j < F.ny - 1 && !(F.mask && F.mask[k]))
             ftle_evec_point(reinterpret_cast<const double2*>(F.out), k, F.ny, F.rdx, F.rdy,
-                            F.rden, ordinary_recip(F.rdx) && ordinary_recip(F.rdy), &fv, &v);
+                            F.rden, ordinary_recips(F.rdx, F.rdy), &fv, &v);
         F.ftle[k] = fv;
         reinterpret_cast<double2*>(F.evec)[k] = v;
     }
@@ -679,10 +686,10 @@ extern "C" int nbcs_ftle_evec_2d(const double* flowmap, int32_t nx, int32_t ny, 
     if (n == 0) return NBCS_OK;
     if (!ftle || !evec_max || (reinterpret_cast<uintptr_t>(evec_max) & 15))
         return set_error(NBCS_ERR_INVALID, "ftle/evec_max NULL or misaligned");
+    const double rdx = 1.0 / (2.0 * dx), rdy = 1.0 / (2.0 * dy);
     ftle_evec_kernel<<<grid_for(n), kStencilThreads, 0, as_stream(stream)>>>(
-        reinterpret_cast<const double2*>(flowmap), nx, fast_div(ny), 1.0 / (2.0 * fabs(T)),
-        1.0 / (2.0 * dx), 1.0 / (2.0 * dy), ordinary_spacing(dx, dy), mask, ftle,
-        reinterpret_cast<double2*>(evec_max));
+        reinterpret_cast<const double2*>(flowmap), nx, fast_div(ny), 1.0 / (2.0 * fabs(T)), rdx,
+        rdy, ordinary_recips(rdx, rdy), mask, ftle, reinterpret_cast<double2*>(evec_max));
     NBCS_LAUNCH_CHECK();
     return NBCS_OK;
 }
