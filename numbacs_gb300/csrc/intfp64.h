@@ -478,17 +478,20 @@ static inline double ip_log(double x)
 }
 
 /* ---- sine and cosine -------------------------------------------------------
- * |x| 2/pi = k + f with k the nearest integer, f in 64-bit fixed point (2/pi to
- * 64 bits); with g = 2 f in [-1, 1] and z = g^2
+ * |x| 2/pi = k + f with k the nearest integer, f in 128-bit fixed point (2/pi to
+ * 128 bits: next to a zero of the sine or the cosine f is as small as the
+ * argument's last bit, and keeps 60 bits of its own there); with g = 2 f in
+ * [-1, 1] and z = g^2
  *   sin(pi/4 g) / (pi/4 g) = 1 - z (q1 - z (q2 - ...)),
  *   cos(pi/4 g)           = 1 - z (c1 - z (c2 - ...)),
  * the Taylor coefficients in units of 2^-64, those below 2^-32 in 32-bit
- * products.  Within 0.52 ulp plus, where the argument is reduced, 2^-58 (what
- * matters next to the zeros other than 0) for |x| < 64; larger arguments, infinities and NaN take the library's. */
+ * products.  Within 0.52 ulp for |x| < 64; larger arguments, infinities and NaN
+ * take the library's. */
 
-/* z and the reduced angle: k, the sign of f and b = 2 |f| */
+/* z and the reduced angle: k, the sign of f and b, b1 = 2 |f| in units of 2^-64
+ * and 2^-128 */
 struct ip_turn {
-    ip_u64 b, z;
+    ip_u64 b, b1, z;
     uint32_t k;     /* quadrant, modulo 4 */
     ip_u64 neg;     /* sign bit of f */
 };
@@ -497,14 +500,19 @@ NBCS_IHD ip_turn ip_reduce(ip_u64 u)
 {
     const int sh = 1075 - ip_exponent(u);  /* 52 - e, in [47, 79] */
     const ip_u64 m = (u & IP_FRACTION) | IP_IMPLICIT;
-    const ip_u64 hi = ip_mulhi(m, 0xa2f9836e4e44152aull), lo = m * 0xa2f9836e4e44152aull;
-    const ip_u64 F = sh < 64 ? (hi << (64 - sh)) | (lo >> sh) : hi >> (sh - 64);
+    const ip_u64 C1 = 0xa2f9836e4e441529ull, C0 = 0xfc2757d1f534ddc0ull;  /* 2/pi */
+    const ip_u64 carry = ip_mulhi(m, C0), lo = m * C0, mid = m * C1 + carry;
+    const ip_u64 hi = ip_mulhi(m, C1) + (mid < carry ? 1u : 0u);
+    /* from 64 on the angle is below pi/4 and nothing is taken from it */
+    const ip_u64 F = sh < 64 ? (hi << (64 - sh)) | (mid >> sh) : hi >> (sh - 64);
+    const ip_u64 F1 = sh < 64 ? (mid << (64 - sh)) | (lo >> sh) : 0ull;
     const uint32_t I = sh < 64 ? (uint32_t)(hi >> sh) : 0u;
     ip_turn t;
     t.neg = F & IP_SIGN;
     t.k = I + (uint32_t)(F >> 63);
-    const ip_u64 a = t.neg ? 0ull - F : F;
-    t.b = (a << 1) - (a >> 63);
+    const ip_u64 a = t.neg ? ~F + (F1 ? 0u : 1u) : F, a1 = t.neg ? 0ull - F1 : F1;
+    t.b = ((a << 1) | (a1 >> 63)) - (a >> 63);
+    t.b1 = a1 << 1;
     t.z = ip_mulhi(t.b, t.b);
     return t;
 }
@@ -546,10 +554,12 @@ NBCS_IHD double ip_sine_of(ip_u64 u, const ip_turn& t)
     ip_u64 A = ip_left(u);
     int e = ip_exponent(u);
     if (t.k) {
-        A = ip_mulhi(t.b, 0xc90fdaa22168c235ull) | 1ull;  /* pi/4 g, units of 2^-64 */
-        const int n = ip_clz64(A);
-        A <<= n;
-        e = 1022 - n;
+        const int n = ip_clz64(t.b | 1ull);  /* |f| is above 2^-62 */
+        /* pi/4 g, units of 2^(-64 - n) */
+        A = ip_mulhi((t.b << n) | ((t.b1 >> 1) >> (63 - n)), 0xc90fdaa22168c235ull);
+        const int up = (int)(A >> 63);
+        A <<= 1 - up;
+        e = 1021 - n + up;
     }
     ip_u64 q = ip_mulhi(A, ip_sine_series(t.z));
     if (!(q >> 63)) {
