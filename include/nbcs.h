@@ -292,11 +292,13 @@ int nbcs_ftle_from_eig(const double* eigval, int64_t n, int64_t stride, double T
 /* Fused C_eig_2D + ftle_from_eig(eigvals[...,1]) + eigvecs[...,:,1]:
  * flowmap -> ftle (nx,ny) and evec_max (nx,ny,2) in one pass (the inputs of
  * ftle_ridge_pts).  The scaling divisions (1/(2dx), 1/(2dy), 1/(2|T|)) are
- * products with reciprocals, the eigenvector is normalised by a reciprocal
- * square root and the log's mantissa part is an FP32 log1p, so the
- * eigenvector is within a few ulp and the FTLE within ~3e-7 relative of
- * nbcs_c_eig_2d + nbcs_ftle_from_eig rather than bit-identical (those two
- * keep the reference's IEEE arithmetic). */
+ * products with reciprocals, the tensor's diagonal, root and eigenvalue are
+ * taken in 64-bit fixed point and the log's mantissa part is an FP32 log1p, so
+ * each component of the eigenvector is within a few ulp of its own (beside what
+ * the tensor's roundings turn the vector by) and the FTLE within ~3e-7 relative
+ * of nbcs_c_eig_2d + nbcs_ftle_from_eig rather than bit-identical (those two
+ * keep the reference's IEEE arithmetic).  A point's results depend on its four
+ * neighbours in the flow map and on nothing else. */
 int nbcs_ftle_evec_2d(const double* flowmap, int32_t nx, int32_t ny, double T, double dx,
                       double dy, const uint8_t* mask, double* ftle, double* evec_max,
                       void* stream);

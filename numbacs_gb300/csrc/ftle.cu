@@ -21,12 +21,12 @@
 // FP64 pipe and as it is: ftle_kernel 401 x 201 23.5 -> 7.9 us, ceig_kernel 1351
 // x 501 with a mask 157 -> 33.6 us, ftle_from_eig_kernel of its eigenvalues 54
 // -> 10 us, ftle_evec_kernel 4001 x 4001 1.87 -> 0.36 ms.  The last, whose
-// roundings are its own, takes fixed point beyond the differences (4 FP64
-// operations a point) and is bound by its 600 instructions a point at 2.75 a
-// cycle; with 14 FP64 sums a point beside integer products it took 0.44 ms (98 %
-// of the FP64 pipe's slots).
+// roundings are its own, takes fixed point for the tensor's diagonal and what
+// follows (eig2_fixed.h; 10 FP64 operations a point); with 14 FP64 sums a point
+// beside integer products it took 0.44 ms (98 % of the FP64 pipe's slots).
 // Compiled with -fmad=false.
 #include "batch_common.cuh"
+#include "eig2_fixed.h"
 #include "intfp64.h"
 #include "nbcs_internal.cuh"
 
@@ -40,10 +40,6 @@ __device__ __forceinline__ bool interior(long k, int nx, const FastDiv& ny, int 
     row_col(k, ny, &i, &j);
     return i >= b && i < nx - b && j >= b && j < (int)ny.d - b;
 }
-
-struct Grad {
-    double dxdx, dxdy, dydx, dydy;
-};
 
 // The arithmetic of a point, FIT when its differences and the grid spacing are
 // ordinary (ordinary_diffs, ordinary_spacing): then every product, quotient and
@@ -340,33 +336,28 @@ __host__ __device__ __forceinline__ bool ordinary_recips(double rdx, double rdy)
 // FP32 pipe: within ~3e-7 relative of ftle_from_eig's where lambda_max >
 // 1 + 1e-6.
 //
-// Nothing here has to repeat the reference's roundings.  In the general form
-// sums of products are one FMA over one product, and the eigenvector is
-// normalised by a reciprocal root instead of a root, a reciprocal and two
-// quotients.
-//
-// Ordinary differences (eigvec_max_fixed) take 64-bit fixed point from the
-// gradients on: the four of them in units of the largest's 2^-62, so that the
-// tensor is four squares' and two products' high halves, whose sums cost a cycle
-// for 19 on the FP64 pipe, with errors below 2^-56 of its largest entry.
+// Ordinary differences (eig2_max_fixed) take 64-bit fixed point from the tensor's
+// diagonal on; its off-diagonal entry, which the vector's smaller component is a
+// multiple of, is the FP64 one in both forms.
 __device__ __forceinline__ double eigvec_max(const Diffs& D, double rdx, double rdy, double* vx,
                                              double* vy)
 {
     using A = Arith<false>;
     const double dxdx = A::mul(D.i.x, rdx), dxdy = A::mul(D.j.x, rdy);
     const double dydx = A::mul(D.i.y, rdx), dydy = A::mul(D.j.y, rdy);
-    const double b = __fma_rn(dxdx, dxdy, A::mul(dydx, dydy));
-    const double a = __fma_rn(dxdx, dxdx, A::mul(dydx, dydx));
-    const double d = __fma_rn(dxdy, dxdy, A::mul(dydy, dydy));
-    const double m = a - d, bb = A::sqr(b);
-    const double disc = A::root(__fma_rn(m, m, A::scale(bb, 2)));
-    const double l1 = A::scale((a + d) + disc, -1);
+    const double b = A::mul(dxdx, dxdy) + A::mul(dydx, dydy);
+    const double a = A::mul(dxdx, dxdx) + A::mul(dydx, dydx);
+    const double d = A::mul(dxdy, dxdy) + A::mul(dydy, dydy);
+    const double l1 = A::scale((a + d) + discriminant<false>(a, b, d), -1);
     const bool age = diag_ge(a, d);
     double ex = age ? 1.0 : 0.0, ey = age ? 0.0 : 1.0;
     if (!ip_zero(b)) {
-        const double e = l1 - (age ? d : a), r = rsqrt(__fma_rn(e, e, bb));
-        ex = (age ? e : b) * r;
-        ey = (age ? b : e) * r;
+        const double e = l1 - (age ? d : a);
+        ex = age ? e : b;
+        ey = age ? b : e;
+        const double r = rsqrt(A::mul(ex, ex) + A::mul(ey, ey));
+        ex *= r;
+        ey *= r;
         positive_x(&ex, &ey);
     }
     *vx = ex;
@@ -374,97 +365,17 @@ __device__ __forceinline__ double eigvec_max(const Diffs& D, double rdx, double 
     return l1;
 }
 
-// a >> n; 0 for n of 64 and more (as the instruction has it)
-__device__ __forceinline__ ip_u64 shifted_right(ip_u64 a, int n)
+// The same of ordinary differences.  Three of the gradients' scalings and b's
+// products on the FP64 pipe beside the integer pipe even the two out: 4001 x 4001
+// 363 us, with all four of them there 382, two 365, none (b's products there)
+// 389, none at all 426.
+__device__ __forceinline__ bool eigvec_max_fit(const Diffs& D, double rdx, double rdy, double* l1,
+                                               double* vx, double* vy)
 {
-    ip_u64 r;
-    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(n));
-    return r;
-}
-
-// a b 2^-64 less the low halves' product: at most two units too small
-__device__ __forceinline__ ip_u64 high_product(ip_u64 a, ip_u64 b)
-{
-    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b,
-                   bh = (uint32_t)(b >> 32);
-    return (ip_u64)ah * bh + (uint32_t)(((ip_u64)al * bh) >> 32) +
-           (uint32_t)(((ip_u64)ah * bl) >> 32);
-}
-
-// the same of factors below 2^63, and the square of one
-__device__ __forceinline__ ip_u64 high_product63(ip_u64 a, ip_u64 b)
-{
-    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b,
-                   bh = (uint32_t)(b >> 32);
-    return (ip_u64)ah * bh + (uint32_t)(((ip_u64)al * bh + (ip_u64)ah * bl) >> 32);
-}
-
-__device__ __forceinline__ ip_u64 high_square63(ip_u64 a)
-{
-    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32);
-    return (ip_u64)ah * ah + (uint32_t)(((ip_u64)ah * al) >> 31);
-}
-
-// The larger eigenvalue's unit vector and the eigenvalue, within two
-// units of the last place.  e = lambda - (smaller diagonal entry) =
-// (|a - d| + disc) / 2 with disc^2 = (a - d)^2 + 4 b^2; the vector is along (e, b)
-// (or (b, e)), whose square length is e disc.
-__device__ __forceinline__ double eigvec_max_fixed(const Diffs& D, double rdx, double rdy,
-                                                   double* vx, double* vy)
-{
-    const ip_u64 rx = ip_bits(rdx), ry = ip_bits(rdy), ix = ip_bits(D.i.x), iy = ip_bits(D.i.y),
-                 jx = ip_bits(D.j.x), jy = ip_bits(D.j.y);
-    // gradients: M 2^-62 2^(e - 2046), M in [2^62, 2^64)
-    const int ex = ip_exponent(rx), ey = ip_exponent(ry);
-    const int e0 = ip_exponent(ix) + ex, e1 = ip_exponent(iy) + ex, e2 = ip_exponent(jx) + ey,
-              e3 = ip_exponent(jy) + ey;
-    const int top = max(max(e0, e1), max(e2, e3)) + 1;
-    const ip_u64 rl = ip_left(rx), sl = ip_left(ry);
-    const ip_u64 p = shifted_right(high_product(ip_left(ix), rl), top - e0),
-                 r = shifted_right(high_product(ip_left(iy), rl), top - e1),
-                 q = shifted_right(high_product(ip_left(jx), sl), top - e2),
-                 s = shifted_right(high_product(ip_left(jy), sl), top - e3);
-    // a, d and b in units of 2^(2 top - 4152)
-    const ip_u64 a = high_square63(p) + high_square63(r), d = high_square63(q) + high_square63(s);
-    const bool opposite = ((ix ^ jx ^ iy ^ jy) >> 63) != 0;
-    const ip_u64 b0 = high_product63(p, q), b1 = high_product63(r, s);
-    const bool less = opposite && b0 < b1;
-    const ip_u64 bm = opposite ? (less ? b1 - b0 : b0 - b1) : b0 + b1;
-    const ip_u64 bsign = ix ^ jx ^ rx ^ ry ^ (less ? IP_SIGN : 0ull);
-    const bool age = a >= d;
-    const ip_u64 m = age ? a - d : d - a, b2 = bm << 1;
-    // disc 2^(z - 1 + h) = root, h 0 or 1
-    const int z = min(ip_clz64(m | b2), 63);
-    const ip_u64 P = m << z, Q = b2 << z;
-    ip_u64 W = high_square63(P >> 1) + high_square63(Q >> 1);
-    const int h = (W >> 62) ? 0 : 1;
-    W <<= 2 * h;
-    const ip_u64 root = ip_root64(W, ip_root_estimate(W));
-    const ip_u64 e = (P >> 2) + (root >> (1 + h));  // e 2^(z - 1)
-    const ip_u64 l = ((age ? d : a) >> 1) + (e >> z);
-    // 1 / sqrt(e disc) = rr 2^(z + h + g - 128)
-    ip_u64 T = high_product(e, root) << h;
-    const int g = (T >> 62) ? 0 : 1;
-    T <<= 2 * g;
-    const ip_u64 rr = ip_rroot64(T, ip_root_estimate(T));
-    double major = 1.0, minor = 0.0;
-    ip_u64 sign = 0;
-    if (b2) {
-        const ip_u64 c = high_product(e, rr) << (h + g);  // units of 2^-63
-        major = ip_double(((c + 0x200ull) >> 10) + (1021ull << 52));
-        const ip_u64 t = high_product(Q, rr);  // units of 2^(h + g - 65)
-        if (t) {
-            const int n = ip_clz64(t);
-            const ip_u64 u = t << n;
-            minor = ip_pack(0, (u >> 11) + ((u >> 10) & 1u), 1023 + 63 - n + h + g - 65);
-            sign = bsign & IP_SIGN;
-        }
-    }
-    const ip_u64 x = ip_bits(age ? major : minor), y = ip_bits(age ? minor : major);
-    *vx = ip_double(x);
-    *vy = ip_double(y | sign);
-    const int n = ip_clz64(l);
-    return ip_pack(0, (l << n) >> 11, 2 * top - 3065 - n);
+    const double dxdx = D.i.x * rdx, dxdy = D.j.x * rdy, dydx = D.i.y * rdx;
+    const double dydy = ip_mul_fit(D.j.y, rdy);
+    const double b = dxdx * dxdy + dydx * dydy;
+    return eig2_max_fixed(dxdx, dxdy, dydx, dydy, b, l1, vx, vy);
 }
 
 // FTLE = log(lambda) / (2|T|) to ~3e-7 relative (the contract is 1e-5):
@@ -495,9 +406,9 @@ __device__ __forceinline__ double ftle_of(double l1, double rden)
         const int z = __clzll((long long)t);
         t <<= z;
         if (ip_fits(ip_bits(rden))) {  // 1 / (2 |T|) is not negative
-            const ip_u64 q = high_product(t, ip_left(ip_bits(rden)));
+            const ip_u64 q = ip_high_product(t, ip_left(ip_bits(rden)));
             const int up = (int)(q >> 63);
-            return ip_pack(0, q >> (10 + up), ip_exponent(ip_bits(rden)) + 9 - z + up);
+            return ip_pack(0, ((q >> (9 + up)) + 1) >> 1, ip_exponent(ip_bits(rden)) + 9 - z + up);
         }
         l = ip_pack(0, (t >> 11) + ((t >> 10) & 1), 1023 + 9 - z);
     }
@@ -511,9 +422,10 @@ __device__ __forceinline__ void ftle_evec_point(const double2* __restrict__ F, l
     const Diffs D = diffs_at(F, k, ny);
     // by the point's own differences (the two forms' last bits differ, and a point
     // has the same result in any row block and any batch)
-    const double l1 = spacing && ordinary_diffs(D.i, D.j)
-                          ? eigvec_max_fixed(D, rdx, rdy, &v->x, &v->y)
-                          : eigvec_max(D, rdx, rdy, &v->x, &v->y);
+    double l1;
+    if (!(spacing && ordinary_diffs(D.i, D.j)) ||
+        !eigvec_max_fit(D, rdx, rdy, &l1, &v->x, &v->y))
+        l1 = eigvec_max(D, rdx, rdy, &v->x, &v->y);
     *f = ftle_of(l1, rden);
 }
 
