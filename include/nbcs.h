@@ -306,7 +306,11 @@ int nbcs_ftle_evec_2d(const double* flowmap, int32_t nx, int32_t ny, double T, d
 /* ------------------------------------------------------------- extraction */
 
 /* np.percentile(f, q) as evaluated in the reference's jitted ftle_ridge_pts
- * (ridges.py:48-51; numba's linear-rank rule), written to *out (device). */
+ * (ridges.py:48-51; numba's linear-rank rule), written to *out (device, or
+ * page-locked host memory).  The launch's blocks wait for one another, each wait
+ * with a limit (about half a second): a launch that gives up writes the NaN of
+ * the bit pattern NBCS_PERCENTILE_FAILED, which no percentile is. */
+#define NBCS_PERCENTILE_FAILED 0x7ff800000000dead
 size_t nbcs_percentile_scratch_bytes(int64_t n);
 int nbcs_percentile(const double* f, int64_t n, double q, double* out, void* scratch,
                     size_t scratch_bytes, void* stream);
@@ -317,7 +321,10 @@ int nbcs_percentile(const double* f, int64_t n, double q, double* out, void* scr
  * points to pts_out (capacity nx*ny rows) and their count to *n_out
  * (int64; like every small result here in device memory or in page-locked
  * host memory, which can be read after a synchronisation).  percentile == 0
- * means threshold 0 (ridges.py:48-49). */
+ * means threshold 0 (ridges.py:48-49).
+ * The launch's blocks wait for one another, each wait with a limit (about half a
+ * second).  A launch that gives up writes -1 to *n_out, 1 to all of mask_out and
+ * NaN to all of rpts_full; pts_out is undefined then. */
 size_t nbcs_ridge_scratch_bytes(int32_t nx, int32_t ny);
 int nbcs_ridge_pts(const double* f, const double* evec_max, const double* x, int32_t nx,
                    const double* y, int32_t ny, double sdd_thresh, double percentile,
@@ -331,7 +338,7 @@ int nbcs_ridge_pts(const double* f, const double* evec_max, const double* x, int
  * point in row-major order) and by row-major order inside each, head[0] the
  * number of points, head[1] that of components and head[2 ..] their sizes
  * (NBCS_RIDGE_COMPONENTS_MAX + 2 int32).  With more points head[1] is -1 and
- * comp_pts is left alone. */
+ * comp_pts is left alone; of a launch that gives up head[0] is -1 too. */
 #define NBCS_RIDGE_COMPONENTS_MAX 8192
 int nbcs_ridge_components(const double* f, const double* evec_max, const double* x, int32_t nx,
                           const double* y, int32_t ny, double sdd_thresh, double percentile,

@@ -30,10 +30,14 @@
 // threshold about half; of all points, percentile 0, 112 us).
 //
 // The barriers wait for blocks of the same cooperative launch only, which the
-// GPU runs all at once, and give up after a fixed number of polls (n_out = -1).
+// GPU runs all at once, and give up after a fixed number of polls.  One block
+// that gives up fails the launch: the others leave at their next poll, and the
+// block that ends last writes the number of points, or -1 and points that are
+// NaN (an atomic a block: 1 us of the launch).
 // Compiled with -fmad=false: the stencil arithmetic is the reference's.
 #include <math.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "intfp64.h"
@@ -49,6 +53,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kCand = 512;        // keys ranked by counting (one per thread)
 constexpr int kKept = 64;         // ridge points a warp keeps; beyond, it evaluates again
 constexpr int kPollLimit = 1 << 20;
+constexpr unsigned kGaveUp = 0x80000000u;
 
 // Scratch; the first part starts at zero (one memset).
 struct SelScratch {
@@ -56,8 +61,9 @@ struct SelScratch {
     unsigned long long above_inv;  // ~(smallest key above the group); 0: none
     unsigned int nan_count, pinf, ninf;
     unsigned int cand_n;
-    unsigned int arrived;          // barrier arrivals
-    unsigned int failed;
+    unsigned int arrived;          // barrier arrivals; kGaveUp: a block has given up
+    unsigned int ended;            // blocks that have written all they will
+    unsigned long long total;      // ridge points, by the last block
     unsigned long long cand[kCand];  // not zeroed
 };
 constexpr size_t kZeroed = offsetof(SelScratch, cand);
@@ -97,6 +103,7 @@ struct RidgeIn {
     int* idx;                // linear indices of the points, or NULL
     int64_t* n_out;
     unsigned int* count;     // ridge points per block
+    int polls;               // after which a barrier gives up
 };
 
 // How the k-th and (k+1)-th order statistics become the percentile (numba's
@@ -112,8 +119,9 @@ struct SelFinish {
 // ------------------------------------------------------------ grid barrier
 
 // Every block of the (cooperative) launch has arrived `phase + 1` times.
-// False, in all threads of the block, when it has waited too long.
-__device__ bool grid_barrier(SelScratch* s, unsigned phase)
+// False, in all threads of the block, when it has waited too long or another
+// block has.
+__device__ bool grid_barrier(SelScratch* s, unsigned phase, int polls)
 {
     __shared__ bool ok;
     __syncthreads();
@@ -121,13 +129,16 @@ __device__ bool grid_barrier(SelScratch* s, unsigned phase)
         __threadfence();
         atomicAdd(&s->arrived, 1u);
         const unsigned want = (phase + 1) * gridDim.x;
-        int polls = 0;
-        unsigned have;
-        do {
+        ok = false;
+        for (; polls > 0; --polls) {
+            unsigned have;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(&s->arrived) : "memory");
-        } while (have < want && ++polls < kPollLimit);
-        ok = have >= want;
-        if (!ok) atomicExch(&s->failed, 1u);
+            if (have >= want) {  // or given up: kGaveUp is above all counts
+                ok = have < kGaveUp;
+                break;
+            }
+        }
+        if (!ok) atomicOr(&s->arrived, kGaveUp);
     }
     __syncthreads();
     return ok;
@@ -176,10 +187,11 @@ struct SelShared {
     double result;
 };
 
-// The percentile of f[0 .. n) in all threads of all blocks (NaN, with *ok false,
-// when a barrier gave up); *phase counts the barriers.
+// The percentile of f[0 .. n) in all threads of all blocks (with *ok false the
+// NaN of a launch that gave up); *phase counts the barriers.
 __device__ double select_percentile(const double* __restrict__ f, long n, SelScratch* s,
-                                    SelShared& sh, const SelFinish& fin, unsigned* phase, bool* ok)
+                                    SelShared& sh, const SelFinish& fin, int polls,
+                                    unsigned* phase, bool* ok)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long stride = (long)gridDim.x * kThreads;
@@ -238,9 +250,9 @@ __device__ double select_percentile(const double* __restrict__ f, long n, SelScr
             if (sh.cnt[1]) atomicAdd(&s->pinf, sh.cnt[1]);
             if (sh.cnt[2]) atomicAdd(&s->ninf, sh.cnt[2]);
         }
-        if (!grid_barrier(s, (*phase)++)) {
+        if (!grid_barrier(s, (*phase)++, polls)) {
             *ok = false;
-            return NAN;
+            return __longlong_as_double((long long)NBCS_PERCENTILE_FAILED);
         }
         // every block: the digit whose cumulative count passes the rank.  Each
         // thread sums four consecutive bins, a block-wide scan of those sums finds
@@ -324,9 +336,9 @@ __device__ double select_percentile(const double* __restrict__ f, long n, SelScr
             for (int w = 1; w < kWarps; ++w) ainv = sh.wmax[w] > ainv ? sh.wmax[w] : ainv;
             if (ainv) atomicMax(&s->above_inv, ainv);
         }
-        if (!grid_barrier(s, (*phase)++)) {
+        if (!grid_barrier(s, (*phase)++, polls)) {
             *ok = false;
-            return NAN;
+            return __longlong_as_double((long long)NBCS_PERCENTILE_FAILED);
         }
     }
     const unsigned long long above = __ldcg(&s->above_inv);
@@ -522,6 +534,66 @@ __device__ __forceinline__ unsigned ridge_run_of(const RidgeIn& R, const RidgeSp
     return found;
 }
 
+// Ridge flags, points and their compaction by a block; false when a barrier gave
+// up.
+__device__ __forceinline__ bool ridge_block(const RidgeIn& R, SelScratch* s, RidgeShared& g,
+                                            double fmin, unsigned phase)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) ridge_spacing(R, &g.S);
+    __syncthreads();
+    // this warp's run of points (whole rounds of 32)
+    const long runs = (long)gridDim.x * kWarps;
+    const long len_all = ((R.n + runs - 1) / runs + 31) / 32 * 32;
+    const long base = ((long)blockIdx.x * kWarps + warp) * len_all;
+    const int len = base >= R.n ? 0 : (int)(R.n - base < len_all ? R.n - base : len_all);
+    RidgeWarp& own = g.w[warp];
+    unsigned long long first = 0;
+    // once for the counts; again, to write, only where a warp has found more
+    // points than it keeps (one copy of the code for both)
+#pragma unroll 1
+    for (int again = 0; again < 2; ++again) {
+        const unsigned found = ridge_run_of(
+            R, g.S, fmin, base, len, !again, own.queue,
+            [&](unsigned rank, int place, double2 p) {
+                if (again) {
+                    R.pts[first + rank] = p;
+                    if (R.idx) R.idx[first + rank] = (int)(base + place);
+                } else if (rank < kKept) {
+                    own.pt[rank] = p;
+                    own.at[rank] = place;
+                }
+            });
+        if (again) break;
+        if (lane == 0) g.wcount[warp] = found;
+        __syncthreads();
+        unsigned total = 0, before = 0;
+        for (int w = 0; w < kWarps; ++w) {
+            if (w < warp) before += g.wcount[w];
+            total += g.wcount[w];
+        }
+        if (tid == 0) R.count[blockIdx.x] = total;
+        if (!grid_barrier(s, phase, R.polls)) return false;
+        // the points of the blocks before this one
+        unsigned long long pre = 0;
+        for (unsigned b = tid; b < blockIdx.x; b += kThreads) pre += __ldcg(R.count + b);
+        for (int o = 16; o > 0; o >>= 1) pre += __shfl_xor_sync(0xffffffffu, pre, o);
+        if (lane == 0) g.wpre[warp] = pre;
+        __syncthreads();
+        for (int w = 0; w < kWarps; ++w) first += g.wpre[w];
+        if (blockIdx.x == gridDim.x - 1 && tid == 0) s->total = first + total;
+        first += before;
+        if (found <= kKept) {
+            for (unsigned q = lane; q < found; q += 32) {
+                R.pts[first + q] = own.pt[q];
+                if (R.idx) R.idx[first + q] = (int)(base + own.at[q]);
+            }
+            break;
+        }
+    }
+    return true;
+}
+
 // One cooperative launch: percentile (when asked for), ridge flags, compaction.
 // RIDGES false: the percentile alone.
 template <bool RIDGES>
@@ -532,74 +604,33 @@ ridge_kernel(RidgeIn R, SelScratch* s, SelFinish fin)
         SelShared sel;
         RidgeShared ridge;
     } sh;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    [[maybe_unused]] __shared__ int end;  // 1: the last block to end, 2: of a launch that failed
+    const int tid = threadIdx.x;
     unsigned phase = 0;
     bool ok = true;
     double fmin = R.fmin_val;
     if (fin.take) {
-        fmin = select_percentile(R.f, R.n, s, sh.sel, fin, &phase, &ok);
+        fmin = select_percentile(R.f, R.n, s, sh.sel, fin, R.polls, &phase, &ok);
+        // (a block that has passed the last barrier has the value, whatever
+        // becomes of the others)
         if (fin.out && blockIdx.x == 0 && tid == 0) *fin.out = fmin;
         __syncthreads();  // the shared memory changes hands
     }
     if constexpr (RIDGES) {
-        if (!ok) {
-            if (blockIdx.x == 0 && tid == 0) *R.n_out = -1;
-            return;
-        }
-        RidgeShared& g = sh.ridge;
-        if (tid == 0) ridge_spacing(R, &g.S);
+        if (ok) ridge_block(R, s, sh.ridge, fmin, phase);
         __syncthreads();
-        // this warp's run of points (whole rounds of 32)
-        const long runs = (long)gridDim.x * kWarps;
-        const long len_all = ((R.n + runs - 1) / runs + 31) / 32 * 32;
-        const long base = ((long)blockIdx.x * kWarps + warp) * len_all;
-        const int len = base >= R.n ? 0 : (int)(R.n - base < len_all ? R.n - base : len_all);
-        RidgeWarp& own = g.w[warp];
-        unsigned long long first = 0;
-        // once for the counts; again, to write, only where a warp has found more
-        // points than it keeps (one copy of the code for both)
-#pragma unroll 1
-        for (int again = 0; again < 2; ++again) {
-            const unsigned found = ridge_run_of(
-                R, g.S, fmin, base, len, !again, own.queue,
-                [&](unsigned rank, int place, double2 p) {
-                    if (again) {
-                        R.pts[first + rank] = p;
-                        if (R.idx) R.idx[first + rank] = (int)(base + place);
-                    } else if (rank < kKept) {
-                        own.pt[rank] = p;
-                        own.at[rank] = place;
-                    }
-                });
-            if (again) return;
-            if (lane == 0) g.wcount[warp] = found;
-            __syncthreads();
-            unsigned total = 0, before = 0;
-            for (int w = 0; w < kWarps; ++w) {
-                if (w < warp) before += g.wcount[w];
-                total += g.wcount[w];
-            }
-            if (tid == 0) R.count[blockIdx.x] = total;
-            if (!grid_barrier(s, phase++)) {
-                if (blockIdx.x == 0 && tid == 0) *R.n_out = -1;
-                return;
-            }
-            // the points of the blocks before this one
-            unsigned long long pre = 0;
-            for (unsigned b = tid; b < blockIdx.x; b += kThreads) pre += __ldcg(R.count + b);
-            for (int o = 16; o > 0; o >>= 1) pre += __shfl_xor_sync(0xffffffffu, pre, o);
-            if (lane == 0) g.wpre[warp] = pre;
-            __syncthreads();
-            for (int w = 0; w < kWarps; ++w) first += g.wpre[w];
-            if (blockIdx.x == gridDim.x - 1 && tid == 0) *R.n_out = (int64_t)(first + total);
-            first += before;
-            if (found <= kKept) {
-                for (unsigned q = lane; q < found; q += 32) {
-                    R.pts[first + q] = own.pt[q];
-                    if (R.idx) R.idx[first + q] = (int)(base + own.at[q]);
-                }
-                return;
-            }
+        if (tid == 0) {
+            __threadfence();
+            end = atomicAdd(&s->ended, 1u) + 1u == gridDim.x ? 1 : 0;
+            __threadfence();
+            if (end && __ldcg(&s->arrived) >= kGaveUp) end = 2;
+            if (end) *R.n_out = end == 2 ? -1 : (int64_t)__ldcg(&s->total);
+        }
+        __syncthreads();
+        if (end != 2) return;
+        for (long k = tid; k < R.n; k += kThreads) {
+            if (R.mask) R.mask[k] = 1;
+            if (R.full) R.full[k] = make_double2(NAN, NAN);
         }
     }
 }
@@ -796,10 +827,19 @@ static SelFinish finish_rule(long n, double q, double* out)
     return fin;
 }
 
+#ifdef NBCS_CHECK
+// the debug library's tests let the barriers give up
+static std::atomic<int> g_polls{kPollLimit};
+static int poll_limit() { return g_polls.load(); }
+#else
+static int poll_limit() { return kPollLimit; }
+#endif
+
 static int launch_ridges(bool ridges, RidgeIn R, SelScratch* s, SelFinish fin, cudaStream_t st)
 {
     unsigned g = ridge_grid(R.n);
     if (g > kMaxBlocks) g = kMaxBlocks;
+    R.polls = poll_limit();
     NBCS_CUDA_TRY(cudaMemsetAsync(s, 0, kZeroed, st));
     void* args[] = {&R, &s, &fin};
     NBCS_CUDA_TRY(cudaLaunchCooperativeKernel(
@@ -812,6 +852,10 @@ static int launch_ridges(bool ridges, RidgeIn R, SelScratch* s, SelFinish fin, c
 }  // namespace nbcs
 
 using namespace nbcs;
+
+#ifdef NBCS_CHECK
+extern "C" void nbcs_check_ridge_polls(int32_t polls) { g_polls.store(polls < 0 ? kPollLimit : polls); }
+#endif
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 

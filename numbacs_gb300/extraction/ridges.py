@@ -24,9 +24,23 @@ def _inputs(f, eigvec_max, x, y):
     return fd, ev, xd, yd
 
 
+# The bit pattern of nbcs_percentile's answer when its launch gave up (nbcs.h)
+_PERCENTILE_FAILED = 0x7ff800000000dead
+
+
+def _count(n_out):
+    """The number of ridge points of a launch that has ended; of one that gave up
+    waiting for its blocks an error."""
+    k = int(n_out)
+    if k < 0:
+        raise RuntimeError("ridge extraction: the launch did not finish")
+    return k
+
+
 def _run(f, eigvec_max, x, y, sdd_thresh, percentile, f_min=None, dxdy=None, full_mask=False):
     """Ridge points (k, 2), or with full_mask (points or zeros (nx*ny, 2), mask
-    (nx, ny)), which are not waited for."""
+    (nx, ny), count), which are not waited for: the caller that waits passes the
+    count to _count (of a launch that gave up the points are NaN, the mask 1)."""
     D.require_cuda()
     fd, ev, xd, yd = _inputs(f, eigvec_max, x, y)
     nx, ny = fd.shape
@@ -49,12 +63,9 @@ def _run(f, eigvec_max, x, y, sdd_thresh, percentile, f_min=None, dxdy=None, ful
                                          D.ptr(full), D.ptr(pts), D.ptr(n_out), D.ptr(scratch),
                                          nbytes, D.stream_ptr()))
     if full_mask:
-        return full, mask
+        return full, mask, n_out
     D.synchronize()
-    k = int(n_out)
-    if k < 0:
-        raise RuntimeError("ridge points: the launch did not finish")
-    return pts[:k]
+    return pts[:_count(n_out)]
 
 
 def ridge_pts_fmin(f, eigvec_max, x, y, dx, dy, sdd_thresh, f_min):
@@ -77,6 +88,8 @@ def percentile(f, q):
     _lib.check(L.nbcs_percentile(D.ptr(fd), fd.numel(), float(q), D.ptr(out), D.ptr(scratch),
                                  nbytes, D.stream_ptr()))
     D.synchronize()
+    if int(out.view(torch.int64)) == _PERCENTILE_FAILED:
+        raise RuntimeError("percentile: the launch did not finish")
     return float(out)
 
 
@@ -89,7 +102,9 @@ def ftle_ridge_pts(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
 def _ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
     """(r_pts (nx*ny, 2) zero off the ridge, ridge_bool (nx, ny), nx, ny)."""
     as_torch = D.is_torch(f, eigvec_max)
-    full, mask = _run(f, eigvec_max, x, y, sdd_thresh, percentile, full_mask=True)
+    full, mask, n_out = _run(f, eigvec_max, x, y, sdd_thresh, percentile, full_mask=True)
+    if not as_torch:
+        _count(n_out)
     nx, ny = mask.shape
     return D.finish(full, as_torch), D.finish(mask.to(torch.bool), as_torch), nx, ny
 
@@ -147,8 +162,7 @@ def ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, min_ridge_pts
     D.synchronize()
     head = head.numpy()
     n, ncomp = int(head[0]), int(head[1])
-    if n < 0:
-        raise RuntimeError("ftle_ridges: the launch did not finish")
+    _count(n)
     if ncomp >= 0:
         counts = head[2:2 + ncomp].tolist()
         pts = comp[:n]

@@ -118,9 +118,10 @@ class GpuOps:
     def ridge_field(self, f, evec, x, y, dx, dy, sdd_thresh, f_min):
         """(ridge mask (n, ny) bool, r_pts (n * ny, 2)) with the threshold and
         spacing given."""
-        from .extraction.ridges import _run
-        full, mask = _run(f, evec, x, y, sdd_thresh, 0, f_min=f_min, dxdy=(dx, dy),
-                          full_mask=True)
+        from .extraction.ridges import _count, _run
+        full, mask, n_out = _run(f, evec, x, y, sdd_thresh, 0, f_min=f_min, dxdy=(dx, dy),
+                                 full_mask=True)
+        _count(n_out)  # block_ridges reads them next
         return mask.to(bool), full
 
     def label8(self, mask):
