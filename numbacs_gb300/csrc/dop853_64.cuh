@@ -371,12 +371,14 @@ __device__ int dop853_solve64(const Flow& fl, const Params& P, double x, double 
     for (;;) {
         if (s0 == 0) {
             if (nstep > nmax) { status = NBCS_PARTICLE_MAX_STEPS; break; }
-            if (dbits(0.1 * abs64(h)) <= dbits(abs64(x) * uround)) {
+            const unsigned long long least = dbits(abs64(x) * uround);
+            // (a NaN on either side, of a NaN start time say, is no underflow)
+            if (dbits(0.1 * abs64(h)) <= least && least <= 0x7ff0000000000000ull) {
                 status = NBCS_PARTICLE_STEP_UNDERFLOW;
                 break;
             }
-            // beyond xend in the direction of the integration
-            if ((long long)(dbits(x + 1.01 * h - xend) ^ sgn) > 0) {
+            // beyond xend in the direction of the integration: above zero, not NaN
+            if ((dbits(x + 1.01 * h - xend) ^ sgn) - 1ull < 0x7ff0000000000000ull) {
                 h = xend - x;
                 last = true;
             }
