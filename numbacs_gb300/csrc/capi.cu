@@ -1,4 +1,5 @@
 // Host-side helpers of the C ABI: error reporting, device queries, flow checks.
+#include <cuda.h>
 #include <stdarg.h>
 #include <stdio.h>
 
@@ -33,6 +34,42 @@ int sm_count()
         cache[dev] = n;
     }
     return cache[dev];
+}
+
+// SMs that kernels of the stream can run on: a green context owns a part of the
+// device's.  Asked of the driver through the runtime, which the library links
+// (0.4 us); where the driver has no answer, the device's.
+int stream_sm_count(cudaStream_t stream)
+{
+    typedef CUresult (*GetCtx)(CUstream, CUcontext*, CUgreenCtx*);
+    typedef CUresult (*GetResource)(CUgreenCtx, CUdevResource*, CUdevResourceType);
+    struct Driver {
+        GetCtx ctx = nullptr;
+        GetResource resource = nullptr;
+        Driver()
+        {
+            void *a = nullptr, *b = nullptr;
+            cudaDriverEntryPointQueryResult r, q;
+            if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &a, 12050, cudaEnableDefault,
+                                                 &r) != cudaSuccess ||
+                cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &b, 12040,
+                                                 cudaEnableDefault, &q) != cudaSuccess ||
+                r != cudaDriverEntryPointSuccess || q != cudaDriverEntryPointSuccess)
+                return;
+            ctx = reinterpret_cast<GetCtx>(a);
+            resource = reinterpret_cast<GetResource>(b);
+        }
+    };
+    static const Driver driver;
+    const int all = sm_count();
+    CUcontext ctx = nullptr;
+    CUgreenCtx green = nullptr;
+    CUdevResource res;
+    if (!driver.ctx || driver.ctx(stream, &ctx, &green) != CUDA_SUCCESS || !green ||
+        driver.resource(green, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return all;
+    const int own = (int)res.sm.smCount;
+    return own >= 1 && own < all ? own : all;
 }
 
 int validate_flow(const nbcs_flow* flow, const double* params, int32_t np, int precision)

@@ -74,6 +74,7 @@ const int g_check_reader_registered = register_check_reader(&read_check_word);
 
 // Number of SMs of the current device (cached per device).
 int sm_count();
+int stream_sm_count(cudaStream_t stream);  // of the stream's context
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -792,13 +792,14 @@ ridge_components_kernel(const double2* __restrict__ pts, const int* __restrict__
     }
 }
 
-// Blocks of a launch: two per SM, all resident at once, and on small fields as
-// few as give every thread four points (a barrier costs by the block: 41, 37
-// and 29 us at one, two and four points a thread on 676 x 251).
-static unsigned ridge_grid(long n)
+// Blocks of a launch: two per SM, all resident at once -- on the SMs that the
+// stream's context owns -- and on small fields as few as give every thread four
+// points (a barrier costs by the block: 41, 37 and 29 us at one, two and four
+// points a thread on 676 x 251).
+static unsigned ridge_grid(long n, cudaStream_t st)
 {
     long b = (n + 4 * kThreads - 1) / (4 * kThreads);
-    const long cap = 2L * sm_count();
+    const long cap = 2L * stream_sm_count(st);
     if (b > cap) b = cap;
     if (b < 1) b = 1;
     return (unsigned)b;
@@ -837,14 +838,21 @@ static int poll_limit() { return kPollLimit; }
 
 static int launch_ridges(bool ridges, RidgeIn R, SelScratch* s, SelFinish fin, cudaStream_t st)
 {
-    unsigned g = ridge_grid(R.n);
+    unsigned g = ridge_grid(R.n, st);
     if (g > kMaxBlocks) g = kMaxBlocks;
     R.polls = poll_limit();
     NBCS_CUDA_TRY(cudaMemsetAsync(s, 0, kZeroed, st));
     void* args[] = {&R, &s, &fin};
-    NBCS_CUDA_TRY(cudaLaunchCooperativeKernel(
-        ridges ? (const void*)ridge_kernel<true> : (const void*)ridge_kernel<false>, dim3(g),
-        dim3(kThreads), args, 0, st));
+    // fewer blocks where that many do not fit at once after all (any number will do)
+    cudaError_t e;
+    do {
+        e = cudaLaunchCooperativeKernel(
+            ridges ? (const void*)ridge_kernel<true> : (const void*)ridge_kernel<false>, dim3(g),
+            dim3(kThreads), args, 0, st);
+        g /= 2;
+        if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();  // not the next call's
+    } while (e == cudaErrorCooperativeLaunchTooLarge && g > 0);
+    NBCS_CUDA_TRY(e);
     NBCS_LAUNCH_CHECK();
     return NBCS_OK;
 }
