@@ -32,8 +32,8 @@
 // The barriers wait for blocks of the same cooperative launch only, which the
 // GPU runs all at once, and give up after a fixed number of polls.  One block
 // that gives up fails the launch: the others leave at their next poll, and the
-// block that ends last writes the number of points, or -1 and points that are
-// NaN (an atomic a block: 1 us of the launch).
+// last block to get past the barriers or to give up writes the number of points,
+// or -1 and points that are NaN (an atomic a block).
 // Compiled with -fmad=false: the stencil arithmetic is the reference's.
 #include <math.h>
 
@@ -62,7 +62,7 @@ struct SelScratch {
     unsigned int nan_count, pinf, ninf;
     unsigned int cand_n;
     unsigned int arrived;          // barrier arrivals; kGaveUp: a block has given up
-    unsigned int ended;            // blocks that have written all they will
+    unsigned int ended;            // blocks past the last barrier, or given up
     unsigned long long total;      // ridge points, by the last block
     unsigned long long cand[kCand];  // not zeroed
 };
@@ -594,6 +594,29 @@ __device__ __forceinline__ bool ridge_block(const RidgeIn& R, SelScratch* s, Rid
     return true;
 }
 
+// A block's warp 0, past the last barrier or after the block has given up: the
+// last of them to come writes the outcome.  (What the blocks write to the mask and
+// the full array they write before that barrier.)
+__device__ __forceinline__ void ridge_end(const RidgeIn& R, SelScratch* s)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned failed = 0;
+    if (lane == 0) {
+        unsigned before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(&s->ended) : "memory");
+        if (before + 1 == gridDim.x) {
+            failed = __ldcg(&s->arrived) >= kGaveUp;
+            *R.n_out = failed ? -1 : (int64_t)__ldcg(&s->total);
+        }
+    }
+    if (!__shfl_sync(0xffffffffu, failed, 0)) return;
+    __syncwarp();
+    for (long k = lane; k < R.n; k += 32) {
+        if (R.mask) R.mask[k] = 1;
+        if (R.full) R.full[k] = make_double2(NAN, NAN);
+    }
+}
+
 // One cooperative launch: percentile (when asked for), ridge flags, compaction.
 // RIDGES false: the percentile alone.
 template <bool RIDGES>
@@ -604,7 +627,6 @@ ridge_kernel(RidgeIn R, SelScratch* s, SelFinish fin)
         SelShared sel;
         RidgeShared ridge;
     } sh;
-    [[maybe_unused]] __shared__ int end;  // 1: the last block to end, 2: of a launch that failed
     const int tid = threadIdx.x;
     unsigned phase = 0;
     bool ok = true;
@@ -618,20 +640,7 @@ ridge_kernel(RidgeIn R, SelScratch* s, SelFinish fin)
     }
     if constexpr (RIDGES) {
         if (ok) ridge_block(R, s, sh.ridge, fmin, phase);
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            end = atomicAdd(&s->ended, 1u) + 1u == gridDim.x ? 1 : 0;
-            __threadfence();
-            if (end && __ldcg(&s->arrived) >= kGaveUp) end = 2;
-            if (end) *R.n_out = end == 2 ? -1 : (int64_t)__ldcg(&s->total);
-        }
-        __syncthreads();
-        if (end != 2) return;
-        for (long k = tid; k < R.n; k += kThreads) {
-            if (R.mask) R.mask[k] = 1;
-            if (R.full) R.full[k] = make_double2(NAN, NAN);
-        }
+        if (tid < 32) ridge_end(R, s);
     }
 }
 
