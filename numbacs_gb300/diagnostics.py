@@ -53,7 +53,9 @@ def ftle_from_eig(eigval_max, T):
     D.require_cuda()
     as_torch = D.is_torch(eigval_max)
     e, stride = eigval_max, 0
-    if isinstance(e, torch.Tensor) and e.is_cuda and e.dtype == torch.float64:
+    # (a lazily negated view -- the imaginary part of a conjugate -- is no plain
+    # memory: its copy is)
+    if isinstance(e, torch.Tensor) and e.is_cuda and e.dtype == torch.float64 and not e.is_neg():
         stride = _step(e)
     if stride == 0:
         e, stride = D.to_dev(e), 1
