@@ -144,11 +144,20 @@ def get_interp_arrays_2D(tvals, xvals, yvals, U, V):
     grid_vel = ((float(tv[0]), float(tv[-1]), nt), (float(xv[0]), float(xv[-1]), nx),
                 (float(yv[0]), float(yv[-1]), ny))
     L = _lib.load()
-    Cu, Cv = D.empty((nt + 2, nx + 2, ny + 2)), D.empty((nt + 2, nx + 2, ny + 2))
+    # both components in the launches of one, for twice the scratch; one after the
+    # other where the device does not have that much
     nbytes = 2 * L.nbcs_spline_prefilter_scratch_bytes(nt, nx, ny)
-    scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=Ud.device)
-    _lib.check(L.nbcs_spline_prefilter_uv(D.ptr(Ud), D.ptr(Vd), nt, nx, ny, D.ptr(Cu), D.ptr(Cv),
-                                          D.ptr(scratch), nbytes, D.stream_ptr()))
+    Cu = Cv = scratch = None
+    try:
+        Cu, Cv = D.empty((nt + 2, nx + 2, ny + 2)), D.empty((nt + 2, nx + 2, ny + 2))
+        scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=Ud.device)
+    except torch.OutOfMemoryError:
+        Cu = Cv = None
+    if scratch is None:
+        Cu, Cv = _prefilter(Ud), _prefilter(Vd)
+    else:
+        _lib.check(L.nbcs_spline_prefilter_uv(D.ptr(Ud), D.ptr(Vd), nt, nx, ny, D.ptr(Cu),
+                                              D.ptr(Cv), D.ptr(scratch), nbytes, D.stream_ptr()))
     return grid_vel, D.finish(Cu, as_torch), D.finish(Cv, as_torch)
 
 
