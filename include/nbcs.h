@@ -75,8 +75,10 @@ typedef struct nbcs_flow {
 typedef struct nbcs_opts {
     int32_t precision;     /* NBCS_PREC_* (default FP64) */
     int32_t max_steps;     /* attempted-step limit per particle (default 100000) */
-    int32_t threads_per_block; /* FP64 path: 0 = library default (128) */
-    int32_t blocks_per_sm;     /* grid cap in blocks per SM; 0 = one block per particle tile */
+    int32_t threads_per_block; /* not used */
+    int32_t blocks_per_sm;     /* grid cap per SM; 0 = one block per particle tile.  Counted in
+                                  blocks of 256 threads (mixed; with a step_model: 128) or of
+                                  256 particles (FP64), whatever the kernels' blocks are */
     int32_t lanes_per_particle; /* mixed spline path: 1, 2 or 4 lanes share a particle; 0 = auto */
     int32_t step_model_mode;    /* how a step_model proposal h_m meets the controller's h_c.
                                    At every fresh step: 0 = h_m, 1 = min(h_m, h_c),

@@ -168,12 +168,7 @@ struct Launch32 {
         using S = TileShape<Flow::LP, kFm32Block, kFm32TileJ>;
         long tiles = (long)((a->nx + S::TI - 1) / S::TI) * ((a->nyv() + S::TJ - 1) / S::TJ);
         long nthreads = tiles * kFm32Block;
-        long blocks = tiles;
-        if (a->blocks_per_sm > 0) {
-            long cap = (long)sm_count() * a->blocks_per_sm;
-            if (blocks > cap) blocks = cap;
-        }
-        if (blocks > (1L << 30)) blocks = 1L << 30;
+        const long blocks = capped_blocks(*a, tiles, kFm32Block);
         flowmap32_kernel<<<(unsigned)blocks, kFm32Block, 0, a->stream>>>(
             fl, to_float(a->P), a->ts, a->te, a->x, a->y, a->nx, a->nyv(), a->aux, a->mask, a->out,
             a->status, a->stats, (float)a->rtol, (float)a->atol, a->nmax, nthreads);

@@ -98,12 +98,9 @@ struct Launch64 {
     {
         using S = TileShape<2, kFm64Block>;
         const int threads = kFm64Block;
-        long blocks = (long)((a->nx + S::TI - 1) / S::TI) * ((a->nyv() + S::TJ - 1) / S::TJ);
-        if (a->blocks_per_sm > 0) {
-            long cap = (long)sm_count() * a->blocks_per_sm;
-            if (blocks > cap) blocks = cap;
-        }
-        if (blocks > (1L << 30)) blocks = 1L << 30;
+        const long blocks = capped_blocks(
+            *a, (long)((a->nx + S::TI - 1) / S::TI) * ((a->nyv() + S::TJ - 1) / S::TJ),
+            S::TI * S::TJ);
         flowmap64_kernel<Flow, FEW><<<(unsigned)blocks, threads, 0, a->stream>>>(
             fl, a->P, a->ts, a->te, a->x, a->y, a->nx, a->nyv(), a->aux, a->mask, a->out,
             a->status, a->stats, a->rtol, a->atol, a->nmax);

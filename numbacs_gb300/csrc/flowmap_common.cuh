@@ -104,6 +104,21 @@ constexpr int kFm32MinBlocks = 6;
 constexpr int kClass32Block = 256;
 constexpr int kClass32MinBlocks = 3;
 
+// blocks_per_sm of a call counts in these units whatever a kernel's own block:
+// 256 threads of the mixed integrators, 256 particles of the FP64 one.  (A limit
+// on what is in flight stays the limit that it was when the blocks shrank.)
+constexpr int kCapUnit = 256;
+
+// blocks of `per_block` threads or particles under the call's cap
+inline long capped_blocks(const FlowmapArgs& a, long blocks, int per_block)
+{
+    if (a.blocks_per_sm > 0) {
+        const long cap = (long)sm_count() * a.blocks_per_sm * (kCapUnit / per_block);
+        if (blocks > cap) blocks = cap;
+    }
+    return blocks > (1L << 30) ? 1L << 30 : blocks;
+}
+
 int launch_flowmap64(const nbcs_flow* flow, const FlowmapArgs& a);
 int launch_flowmap32(const nbcs_flow* flow, const FlowmapArgs& a);
 int launch_flowmap32_learned(const nbcs_flow* flow, const FlowmapArgs& a, int mode);

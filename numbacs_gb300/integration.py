@@ -50,8 +50,9 @@ def flowmap_grid_2D(funcptr, t0, T, x, y, params, method="dop853", rtol=1e-6, at
     accepted / rejected / RHS-evaluation counts), ``out`` (a preallocated
     (nx, ny, 2) float64 CUDA tensor), and the launch-shape knobs
     ``lanes_per_particle`` (mixed spline path: 1, 2 or 4 lanes share one
-    particle's RHS; 0 = automatic) and ``blocks_per_sm`` (0 = one block per
-    particle tile).  ``step_model`` (a learned.StepProposer; mixed precision,
+    particle's RHS; 0 = automatic) and ``blocks_per_sm`` (a cap on what is in
+    flight, in units of 256 threads for "mixed" and of 256 particles for "fp64";
+    0 = one block per particle tile).  ``step_model`` (a learned.StepProposer; mixed precision,
     spline flows) proposes each step from local flow features, and
     ``step_model_mode`` combines its proposal h_m with the controller's h_c
     (0: h_m, 1: min(h_m, h_c), 2: sqrt(h_m h_c)).
