@@ -708,10 +708,14 @@ ridge_components_kernel(const double2* __restrict__ pts, const int* __restrict__
     }
     __syncthreads();
     // Shiloach & Vishkin (1982): shorten all paths to stars by pointer jumping,
-    // hook the larger of two touching stars' roots to the smaller, until nothing
-    // changes (each round at least halves the stars that touch another)
-    for (int round = 0; round < 16; ++round) {
-        for (int jump = 0; jump < 16; ++jump) {
+    // hook the larger of two touching stars' roots to the smaller, until no two
+    // touch.  Of touching stars at least one root a round is hooked, so the rounds
+    // end; a star that nothing hooks to and that stays in one round (its neighbours
+    // found smaller ones) is hooked itself in the next, so two rounds leave at most
+    // half of a component's stars; a handful of rounds do for ridges, up to 11 for
+    // combs of 8192 points.  A path of 8192 links is short after 13 jumps.
+    for (int round = 0; round < kCompMax; ++round) {
+        for (int jump = 0; jump < 14; ++jump) {
             int moved = 0;
             for (int q = tid; q < n; q += kCompThreads) {
                 const int p = parent[q], g = parent[p];
