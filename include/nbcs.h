@@ -240,8 +240,9 @@ int nbcs_batch_prepare(const nbcs_flow* flows, int32_t nflows, const nbcs_field*
  * of all fields in one launch.  Kernel launches only: capturable in a CUDA
  * graph.  Two schedules, chosen by opts->blocks_per_sm:
  *   >= 0  one persistent grid of blocks_per_sm blocks per SM (0 = full
- *         occupancy) whose warps take 32-particle chunks of any field from a
- *         shared counter;
+ *         occupancy; a block is 128 threads, of an FP64 plan 128 particles)
+ *         whose warps take 32-particle chunks of any field from a shared
+ *         counter;
  *   <  0  (mixed precision) per flow class one launch of that class's tile
  *         kernel -- the single-field integrator's block shape and register
  *         budget -- with one block per particle tile of the class's fields,

@@ -70,7 +70,8 @@ int launch_batch64(const BatchHeader* dev_hdr, const DevFlow64* flows, const Dev
     BatchHeader* hdr = const_cast<BatchHeader*>(dev_hdr);
     batch64_reset_kernel<<<1, 1, 0, s>>>(hdr);
     NBCS_LAUNCH_CHECK();
-    int per_sm = blocks_per_sm;
+    // a caller's block is kBatchThreads particles in flight, two lanes each here
+    int per_sm = 2 * blocks_per_sm;
     if (per_sm <= 0 &&
         (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch64_kernel, kBatchThreads, 0) !=
              cudaSuccess ||
