@@ -68,6 +68,41 @@ def _jsonable(o):
     raise TypeError("not JSON serialisable: %r" % type(o))
 
 
+# What the printed line keeps of a long table's rows (the whole of them: --detail).
+# With every figure of every row the line was 36 KB, and a runner that keeps the
+# last 30 KB of a program's output did not find its beginning.
+_LADDER_KEYS = ("precision", "rtol", "atol", "flowmap_ms", "mean", "q99", "max")
+_SWEEP_KEYS = ("field", "rtol", "atol", "particles", "mixed_vs_fp64_max", "mixed_vs_fp64_mean",
+               "mixed_ms", "fp64_ms", "speedup")
+
+
+def _rounded(v, digits=6):
+    """v with the floats inside its containers to `digits` significant digits"""
+    if isinstance(v, dict):
+        return {k: _rounded(x, digits) for k, x in v.items()}
+    if isinstance(v, (list, tuple, set)):
+        return [_rounded(x, digits) for x in v]
+    if hasattr(v, "item"):
+        v = v.item()
+    return float("%.*g" % (digits, v)) if isinstance(v, float) else v
+
+
+def line_of(out):
+    """The result as the one printed line: the headline and the end-to-end figures in
+    full, the legs' to six digits, the rows of the two long tables cut to what is read
+    in them."""
+    short = dict(out)
+    for k, v in out.items():
+        if isinstance(v, (dict, list)) and k not in ("config", "e2e", "clocks"):
+            short[k] = _rounded(v)
+    pick = lambda rows, keys: [{k: r[k] for k in keys if k in r} for r in rows]  # noqa: E731
+    if isinstance(short.get("accuracy"), dict) and "ladder" in short["accuracy"]:
+        short["accuracy"]["ladder"] = pick(short["accuracy"]["ladder"], _LADDER_KEYS)
+    if isinstance(short.get("c3_precision_sweep"), list):
+        short["c3_precision_sweep"] = pick(short["c3_precision_sweep"], _SWEEP_KEYS)
+    return json.dumps(short, default=_jsonable)
+
+
 _T_START = time.perf_counter()
 
 
@@ -112,6 +147,8 @@ def parse():
                     choices=["ftle", "ridge", "compose", "label", "batch", "mlp", "stencils", "aux",
                              "prefilter", "learned"],
                     help="run one small case of one kernel family 3 times (for ncu captures)")
+    ap.add_argument("--detail", default=None, metavar="FILE",
+                    help="also write the whole result, every row of every table, to FILE")
     ap.add_argument("--quick", action="store_true",
                     help="timed steps only (no ladder, plain comparison, e2e or CPU baseline)")
     return ap.parse_args()
@@ -1346,7 +1383,10 @@ def main():
     rank, world, _ = dist_setup()
     out = run_ours(args, rank, world)
     if rank == 0:
-        print(json.dumps(out, default=_jsonable))
+        if args.detail:
+            with open(args.detail, "w") as fh:
+                json.dump(out, fh, default=_jsonable)
+        print(line_of(out))
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
