@@ -6,16 +6,18 @@
  * division in 137, a square root in 143 and log() in about 570; a 32-bit
  * integer or logic instruction takes half a cycle and the high half of a
  * 64 x 64-bit product 4.3 (all measured).  The operations below work on the
- * 53-bit significands in 64-bit registers: about 15 cycles for a product, 13
- * for a quotient whose divisor's reciprocal is at hand, 25 for a reciprocal or
- * a square root, 35 for a logarithm, and they run beside the FP64 pipe.
+ * 53-bit significands in 64-bit registers: 13 cycles for a product (15 with the
+ * test of the operands' ranges), 17 for a quotient whose divisor's reciprocal is
+ * at hand, 34 for one with the reciprocal, 27 for a square root, 53 for a
+ * logarithm, 115 for a sine and cosine (the library's: 438), and they run beside
+ * the FP64 pipe.
  *
  * ip_mul, ip_div and ip_sqrt are correctly rounded (round to nearest even): the
  * same bits as * / sqrt.  The product is exact in 106 bits.  Quotient and root
  * come from a hardware FP32 estimate and two Newton-Raphson corrections in
  * fixed point (64 bits, a few units off); where those units could change the
  * rounding, the midpoint itself is multiplied back and compared.  ip_log is
- * within 0.65 ulp (a table of 128 reciprocals, after P. T. P. Tang's
+ * within 0.55 ulp (a table of 128 reciprocals, after P. T. P. Tang's
  * table-driven logarithm, 1990, with log1p of the exact remainder by its
  * Taylor series in fixed point).
  *
@@ -488,33 +490,46 @@ static inline double ip_log(double x)
  * products.  Within 0.52 ulp for |x| < 64; larger arguments, infinities and NaN
  * take the library's. */
 
-/* z and the reduced angle: k, the sign of f and b, b1 = 2 |f| in units of 2^-64
- * and 2^-128 */
+/* k, the sign of f and z = (2 f)^2 from 2/pi to 64 bits (rounded: f within two
+ * units of 2^-64, which the series do not notice; |f| is above 2^-62 for every
+ * double of this range that is reduced, so the sign is right) */
 struct ip_turn {
-    ip_u64 b, b1, z;
-    uint32_t k;     /* quadrant, modulo 4 */
-    ip_u64 neg;     /* sign bit of f */
+    ip_u64 hi, lo, z;  /* m 2/pi in units of 2^(e - 116), m 2^(e - 52) the argument */
+    uint32_t k;        /* quadrant, modulo 4 */
+    ip_u64 neg;        /* sign bit of f */
 };
 
 NBCS_IHD ip_turn ip_reduce(ip_u64 u)
 {
     const int sh = 1075 - ip_exponent(u);  /* 52 - e, in [47, 79] */
     const ip_u64 m = (u & IP_FRACTION) | IP_IMPLICIT;
-    const ip_u64 C1 = 0xa2f9836e4e441529ull, C0 = 0xfc2757d1f534ddc0ull;  /* 2/pi */
-    const ip_u64 carry = ip_mulhi(m, C0), lo = m * C0, mid = m * C1 + carry;
-    const ip_u64 hi = ip_mulhi(m, C1) + (mid < carry ? 1u : 0u);
-    /* from 64 on the angle is below pi/4 and nothing is taken from it */
-    const ip_u64 F = sh < 64 ? (hi << (64 - sh)) | (mid >> sh) : hi >> (sh - 64);
-    const ip_u64 F1 = sh < 64 ? (mid << (64 - sh)) | (lo >> sh) : 0ull;
-    const uint32_t I = sh < 64 ? (uint32_t)(hi >> sh) : 0u;
     ip_turn t;
+    t.hi = ip_mulhi(m, 0xa2f9836e4e44152aull);
+    t.lo = m * 0xa2f9836e4e44152aull;
+    const ip_u64 F = sh < 64 ? (t.hi << (64 - sh)) | (t.lo >> sh) : t.hi >> (sh - 64);
+    const uint32_t I = sh < 64 ? (uint32_t)(t.hi >> sh) : 0u;
     t.neg = F & IP_SIGN;
     t.k = I + (uint32_t)(F >> 63);
-    const ip_u64 a = t.neg ? ~F + (F1 ? 0u : 1u) : F, a1 = t.neg ? 0ull - F1 : F1;
-    t.b = ((a << 1) | (a1 >> 63)) - (a >> 63);
-    t.b1 = a1 << 1;
-    t.z = ip_mulhi(t.b, t.b);
+    const ip_u64 a = t.neg ? 0ull - F : F, b = (a << 1) - (a >> 63);
+    t.z = ip_mulhi(b, b);
     return t;
+}
+
+/* 2 |f| with 2/pi to 128 bits (the 64 bits above less 2^-128 of the constant
+ * below), for an argument with k: shifted up to bit 63, *n places from units of
+ * 2^-64 */
+NBCS_IHD ip_u64 ip_angle(ip_u64 u, const ip_turn& t, int* n)
+{
+    const int sh = 1075 - ip_exponent(u);  /* in [47, 53] */
+    const ip_u64 m = (u & IP_FRACTION) | IP_IMPLICIT;
+    const ip_u64 low = 0ull - m * 0x03d8a82e0acb2240ull;
+    const ip_u64 less = ip_mulhi(m, 0x03d8a82e0acb2240ull) + (low ? 1u : 0u);
+    const ip_u64 mid = t.lo - less, hi = t.hi - (t.lo < less ? 1u : 0u);
+    const ip_u64 F = (hi << (64 - sh)) | (mid >> sh), F1 = (mid << (64 - sh)) | (low >> sh);
+    const ip_u64 a = t.neg ? ~F + (F1 ? 0u : 1u) : F, a1 = t.neg ? 0ull - F1 : F1;
+    const int z = ip_clz64(a | 1ull);
+    *n = z - 1;
+    return (a << z) | ((a1 >> 1) >> (63 - z));
 }
 
 /* 1 - z (q1 - ...) in units of 2^-64, below 1 */
@@ -554,9 +569,8 @@ NBCS_IHD double ip_sine_of(ip_u64 u, const ip_turn& t)
     ip_u64 A = ip_left(u);
     int e = ip_exponent(u);
     if (t.k) {
-        const int n = ip_clz64(t.b | 1ull);  /* |f| is above 2^-62 */
-        /* pi/4 g, units of 2^(-64 - n) */
-        A = ip_mulhi((t.b << n) | ((t.b1 >> 1) >> (63 - n)), 0xc90fdaa22168c235ull);
+        int n;
+        A = ip_mulhi(ip_angle(u, t, &n), 0xc90fdaa22168c235ull);  /* units of 2^(-64 - n) */
         const int up = (int)(A >> 63);
         A <<= 1 - up;
         e = 1021 - n + up;
