@@ -32,7 +32,7 @@
 // Flow maps with one lane a particle and all arithmetic on the FP64 pipe, and
 // as it is: double gyre 401 x 201 5.45 -> 2.75 ms, 21 x 11 1.02 -> 0.64 ms;
 // geophysical flow 338 x 126 at rtol 1e-6 31.3 -> 22.1 ms, where the FP64 pipe
-// is busy 84 % of the time (143 operations an evaluation and lane pair).
+// is busy 79 % of the time (143 operations an evaluation and lane pair).
 //
 // Code shape: integer arithmetic is many instructions, and what a step runs
 // through has to stay in the instruction caches (with the stage sums unrolled

@@ -90,17 +90,17 @@ struct FlowmapArgs {
 // neighbouring trajectories; smaller blocks share out a grid of a few blocks per
 // SM more evenly and leave their place sooner when a trajectory lags.  Geophysical
 // flow map (rtol 3e-9) with 256-thread 16 x 8, 128-thread 8 x 8 and 64-thread 8 x 4
-// tiles: 338 x 126 particles 2.92, 2.67 and 2.78 ms, 676 x 251 6.70, 6.65 and
-// (rtol 1e-7) 3.68, 3.68 and 3.96 ms, 1351 x 501 21.4 and 21.3 ms; double gyre
-// 401 x 201 134, 120 and 119 us.  The minimum of 6 resident blocks gives the
+// tiles: 338 x 126 particles 2.92, 2.67 and 2.78 ms; larger grids the same within
+// a run's noise, but for the third (676 x 251 at rtol 1e-7 3.68, 3.68 and 3.96 ms);
+// double gyre 401 x 201 134, 120 and 119 us.  The minimum of 6 resident blocks gives the
 // compiler 85 registers a thread; it takes 80 with no spills (24 warps per SM).
 constexpr int kFm32Block = 128;
 constexpr int kFm32TileJ = 8;
 constexpr int kFm32MinBlocks = 6;
 
 // The same of the batch's class launches, whose many blocks share the SMs evenly
-// anyway: six geophysical fields and a jet 23.1 ms with 256-thread blocks, 24.1
-// with 128.
+// anyway: six geophysical fields and a jet in turn 23.1 ms with 256-thread blocks,
+// 24.1 with 128.
 constexpr int kClass32Block = 256;
 constexpr int kClass32MinBlocks = 3;
 

@@ -15,7 +15,7 @@
 // warp, 137 for a division, 143 for a square root, 570 for log(), against
 // some 35 cycles of HBM time for a warp's points.  So the products, quotients,
 // roots and logarithms run on the integer pipe (intfp64.h: correctly rounded,
-// the same bits; about 15, 13, 25 and 35 cycles) and only the sums, which an
+// the same bits; about 13, 17, 27 and 53 cycles) and only the sums, which an
 // integer pipe does not do faster, stay on the FP64 pipe beside it (and a pair
 // of products, to even out the two pipes).  Kernel times with everything on the
 // FP64 pipe and as it is: ftle_kernel 401 x 201 23.5 -> 7.9 us, ceig_kernel 1351
