@@ -55,7 +55,7 @@ def ftle_ordered_ridges(f, eigvec_max, x, y, dist_tol, ep_tan_ang=math.pi / 4, m
     """Ordered FTLE ridge curves (a list of (m, 2) arrays), same signature and
     defaults as the reference; the ridge test runs on the GPU."""
     from .ridges import _ftle_ridges
-    r_full, mask, _, _ = _ftle_ridges(f, eigvec_max, x, y, sdd_thresh, percentile)
+    r_full, mask, _, _ = _ftle_ridges(f, eigvec_max, x, y, sdd_thresh, percentile, wait=True)
     if hasattr(mask, "cpu"):
         mask, r_full = mask.cpu().numpy(), r_full.cpu().numpy()
     fh = f.cpu().numpy() if hasattr(f, "cpu") else f

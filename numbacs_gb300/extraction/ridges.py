@@ -99,11 +99,13 @@ def ftle_ridge_pts(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
     return D.finish(_run(f, eigvec_max, x, y, sdd_thresh, percentile), as_torch)
 
 
-def _ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0):
-    """(r_pts (nx*ny, 2) zero off the ridge, ridge_bool (nx, ny), nx, ny)."""
+def _ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, *, wait=False):
+    """(r_pts (nx*ny, 2) zero off the ridge, ridge_bool (nx, ny), nx, ny).  Torch
+    callers are not waited for unless they say so (a launch that gave up then raises,
+    as for numpy callers)."""
     as_torch = D.is_torch(f, eigvec_max)
     full, mask, n_out = _run(f, eigvec_max, x, y, sdd_thresh, percentile, full_mask=True)
-    if not as_torch:
+    if wait or not as_torch:
         _count(n_out)
     nx, ny = mask.shape
     return D.finish(full, as_torch), D.finish(mask.to(torch.bool), as_torch), nx, ny

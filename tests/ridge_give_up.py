@@ -13,6 +13,7 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import numbacs_gb300 as nb  # noqa: E402
 from numbacs_gb300 import _lib, shard  # noqa: E402
 from numbacs_gb300.extraction import _ftle_ridges, ftle_ridge_pts, ftle_ridges  # noqa: E402
+from numbacs_gb300.extraction.ordered import ftle_ordered_ridges  # noqa: E402
 from numbacs_gb300.extraction.ridges import percentile, ridge_pts_fmin  # noqa: E402
 
 
@@ -34,6 +35,8 @@ def main():
         "pts, no percentile": lambda: ftle_ridge_pts(f, e, x, y, 0.0, 0),
         "fmin": lambda: ridge_pts_fmin(f, e, x, y, 0.5, 0.25, 0.0, 5.5),
         "ridges": lambda: np.concatenate(ftle_ridges(f, e, x, y, 0.0, 95)),
+        "ordered torch": lambda: np.concatenate(
+            [np.zeros((0, 2))] + ftle_ordered_ridges(*dev, 1.0, min_ridge_pts=1, percentile=99)),
         "field": lambda: _ftle_ridges(f, e, x, y, 0.0, 90)[0],
         "shard": lambda: ops.ridge_field(f, e, x, y, 0.5, 0.25, 0.0, 5.5)[1].cpu().numpy(),
     }
