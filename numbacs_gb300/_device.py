@@ -87,7 +87,9 @@ def empty(shape, dtype=torch.float64):
 def readback(shape, dtype):
     """Page-locked host array that a kernel writes and the host reads after
     synchronize(): a small result without a device-to-host copy behind the
-    kernel (7 us less per call).  Synchronize before it goes out of scope."""
+    kernel (7 us less per call).  Synchronize before it goes out of scope, also
+    where the call that may have launched the kernel raises: the allocator hands
+    the memory out again at once."""
     return torch.empty(shape, dtype=dtype, pin_memory=True)
 
 

@@ -51,20 +51,23 @@ def _run(f, eigvec_max, x, y, sdd_thresh, percentile, f_min=None, dxdy=None, ful
     full = D.empty((nx * ny, 2)) if full_mask else None
     pts = D.empty((nx * ny, 2))
     n_out = D.empty((1,), torch.int64) if full_mask else D.readback((1,), torch.int64)
-    if f_min is None:
-        _lib.check(L.nbcs_ridge_pts(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
-                                    float(sdd_thresh), float(percentile), D.ptr(mask),
-                                    D.ptr(full), D.ptr(pts), D.ptr(n_out), D.ptr(scratch), nbytes,
-                                    D.stream_ptr()))
-    else:
-        _lib.check(L.nbcs_ridge_pts_fmin(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
-                                         float(dxdy[0]), float(dxdy[1]), float(sdd_thresh),
-                                         float(f_min), D.ptr(mask),
-                                         D.ptr(full), D.ptr(pts), D.ptr(n_out), D.ptr(scratch),
-                                         nbytes, D.stream_ptr()))
+    try:
+        if f_min is None:
+            _lib.check(L.nbcs_ridge_pts(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
+                                        float(sdd_thresh), float(percentile), D.ptr(mask),
+                                        D.ptr(full), D.ptr(pts), D.ptr(n_out), D.ptr(scratch),
+                                        nbytes, D.stream_ptr()))
+        else:
+            _lib.check(L.nbcs_ridge_pts_fmin(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
+                                             float(dxdy[0]), float(dxdy[1]), float(sdd_thresh),
+                                             float(f_min), D.ptr(mask), D.ptr(full), D.ptr(pts),
+                                             D.ptr(n_out), D.ptr(scratch), nbytes,
+                                             D.stream_ptr()))
+    finally:
+        if not full_mask:
+            D.synchronize()  # n_out is page-locked: also when the call raised
     if full_mask:
         return full, mask, n_out
-    D.synchronize()
     return pts[:_count(n_out)]
 
 
@@ -85,9 +88,11 @@ def percentile(f, q):
     nbytes = L.nbcs_percentile_scratch_bytes(fd.numel())
     scratch = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=fd.device)
     out = D.readback((1,), torch.float64)
-    _lib.check(L.nbcs_percentile(D.ptr(fd), fd.numel(), float(q), D.ptr(out), D.ptr(scratch),
-                                 nbytes, D.stream_ptr()))
-    D.synchronize()
+    try:
+        _lib.check(L.nbcs_percentile(D.ptr(fd), fd.numel(), float(q), D.ptr(out), D.ptr(scratch),
+                                     nbytes, D.stream_ptr()))
+    finally:
+        D.synchronize()
     if int(out.view(torch.int64)) == _PERCENTILE_FAILED:
         raise RuntimeError("percentile: the launch did not finish")
     return float(out)
@@ -157,11 +162,13 @@ def ftle_ridges(f, eigvec_max, x, y, sdd_thresh=0.0, percentile=0, min_ridge_pts
     cap = _lib.RIDGE_COMPONENTS_MAX
     comp = D.empty((cap, 2))
     head = D.readback((cap + 2,), torch.int32)
-    _lib.check(L.nbcs_ridge_components(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
-                                       float(sdd_thresh), float(percentile), D.ptr(mask),
-                                       D.ptr(pts), D.ptr(index), D.ptr(n_out), D.ptr(comp),
-                                       D.ptr(head), D.ptr(scratch), nbytes, D.stream_ptr()))
-    D.synchronize()
+    try:
+        _lib.check(L.nbcs_ridge_components(D.ptr(fd), D.ptr(ev), D.ptr(xd), nx, D.ptr(yd), ny,
+                                           float(sdd_thresh), float(percentile), D.ptr(mask),
+                                           D.ptr(pts), D.ptr(index), D.ptr(n_out), D.ptr(comp),
+                                           D.ptr(head), D.ptr(scratch), nbytes, D.stream_ptr()))
+    finally:
+        D.synchronize()
     head = head.numpy()
     n, ncomp = int(head[0]), int(head[1])
     _count(n)
