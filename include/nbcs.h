@@ -467,12 +467,10 @@ int nbcs_ridge_pts_noalloc(const double* f, const double* evec_max, const double
 #define NBCS_CHECK_LABEL_LINK 0x4u
 int nbcs_check_enabled(void);
 int nbcs_check_bits(uint32_t* bits, int32_t reset);
-/* That build alone also has nbcs_check_ridge_polls(int32_t polls): after how many
- * polls a grid-wide wait of the ridge launches gives up (below 0: the usual limit),
- * so that a test can make waits run out. */
-#ifdef NBCS_CHECK
-void nbcs_check_ridge_polls(int32_t polls);
-#endif
+/* After how many polls a grid-wide wait of the ridge launches gives up (below 0:
+ * the usual limit), so that a test can make waits run out: in that build only,
+ * NBCS_ERR_UNSUPPORTED in the normal one. */
+int nbcs_check_ridge_polls(int32_t polls);
 
 /* Number of kernels this library has launched in the process so far. */
 unsigned long long nbcs_launch_count(void);

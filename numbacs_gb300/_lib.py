@@ -135,6 +135,7 @@ SIGNATURES = {
     "nbcs_launch_count": (ctypes.c_ulonglong, []),
     "nbcs_check_enabled": (ctypes.c_int, []),
     "nbcs_check_bits": (ctypes.c_int, [ctypes.POINTER(ctypes.c_uint32), _i32]),
+    "nbcs_check_ridge_polls": (ctypes.c_int, [_i32]),
     "nbcs_probe_fma": (ctypes.c_int, [_i32, _i64, _vp, ctypes.POINTER(ctypes.c_double), _vp]),
 }
 

@@ -874,9 +874,16 @@ static int launch_ridges(bool ridges, RidgeIn R, SelScratch* s, SelFinish fin, c
 
 using namespace nbcs;
 
+extern "C" int nbcs_check_ridge_polls(int32_t polls)
+{
 #ifdef NBCS_CHECK
-extern "C" void nbcs_check_ridge_polls(int32_t polls) { g_polls.store(polls < 0 ? kPollLimit : polls); }
+    g_polls.store(polls < 0 ? kPollLimit : polls);
+    return NBCS_OK;
+#else
+    (void)polls;
+    return set_error(NBCS_ERR_UNSUPPORTED, "check_ridge_polls: the bounds-checked build only");
 #endif
+}
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 

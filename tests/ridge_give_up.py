@@ -43,7 +43,7 @@ def main():
     want = {k: c() for k, c in calls.items()}
     given_up = finished = 0
     for polls in [0] + [1, 2, 4, 8, 16, 32, 64, 128, 256, 1024] * 8:
-        L.nbcs_check_ridge_polls(polls)
+        _lib.check(L.nbcs_check_ridge_polls(polls))
         for name, call in calls.items():
             try:
                 got = call()
@@ -58,7 +58,7 @@ def main():
         full, mask = full.cpu().numpy(), mask.cpu().numpy()
         assert polls or np.isnan(full).all()
         assert (np.isnan(full).all() and mask.all()) or np.array_equal(full, want["field"])
-    L.nbcs_check_ridge_polls(-1)
+    _lib.check(L.nbcs_check_ridge_polls(-1))
     for name, call in calls.items():
         assert np.array_equal(call(), want[name]), name
     print("gave up: all at no polls, %d in all; finished: %d" % (given_up, finished))
